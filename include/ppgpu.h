@@ -113,8 +113,9 @@ int ppgpu_pack_atoms(int natoms, const double *R, const double *cLJ, const doubl
 #define PPGPU_FF_QZS 3
 #define PPGPU_FF_WITH_E 1
 #define PPGPU_FF_ACCUMULATE 2
-#define PPGPU_FF_F64 4 /* evaluate the sums in float64 (the GPU error oracle); always on for
-                          the pz/dz2 Coulomb tips, whose finite differences need it */
+#define PPGPU_FF_F64 4 /* evaluate the sums in float64 (the GPU error oracle); without it the
+                          pz/dz2 Coulomb tips, whose finite differences cancel, run in
+                          double-float and round like it */
 int ppgpu_ff_grid(float *FE, const int *n, const double *cell, const float *atoms, int natoms, int ncharged,
                   int mode, int coul_kind, double Q, double Fmax, const double *Qs, const double *QZs, int flags,
                   void *stream);
