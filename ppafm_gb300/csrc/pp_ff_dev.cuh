@@ -49,6 +49,11 @@ inline void ff_set_offsets(FFParams &prm) {
         for (int i = 0; i < FF_MAX_P; i++) prm.off[c][i] = (float)(prm.dC[c] * i);
 }
 
+// Force fields by boxes (pp_ff_box.cu): whether a grid and its atoms are summed that way, with
+// how many levels of boxes above the leaves, and the launch.
+bool ff_box_rule(const FFParams &prm, int mode, int *levels);
+int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, int levels, cudaStream_t st);
+
 // ------------------------------------------------------------------ TMA helpers
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
