@@ -56,6 +56,17 @@ __device__ __forceinline__ dfl df_mul(dfl a, dfl b) {
     return fast_two_sum(p.h, e);
 }
 
+// a * b without the final renormalisation: the low part stays below 2^-21 of the high one.
+__device__ __forceinline__ dfl df_mul_raw(dfl a, dfl b) {
+    const dfl p = two_prod(a.h, b.h);
+    return {p.h, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, p.l))};
+}
+
+__device__ __forceinline__ dfl df_mul_raw(dfl a, float b) {
+    const dfl p = two_prod(a.h, b);
+    return {p.h, __fmaf_rn(a.l, b, p.l)};
+}
+
 __device__ __forceinline__ dfl df_mul_f(dfl a, float b) {
     const dfl p = two_prod(a.h, b);
     return fast_two_sum(p.h, __fmaf_rn(a.l, b, p.l));

@@ -217,17 +217,6 @@ static int ff64_dispatch(const FFParams &prm, int mode, int kind, cudaStream_t s
 constexpr int TIP_P = 4;
 constexpr int TIP_THREADS = 128;
 
-// a * b without the final renormalisation (the low part stays below 2^-21 of the high one).
-__device__ __forceinline__ dfl df_mul_raw(dfl a, dfl b) {
-    const dfl p = two_prod(a.h, b.h);
-    return {p.h, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, p.l))};
-}
-
-__device__ __forceinline__ dfl df_mul_raw(dfl a, float b) {
-    const dfl p = two_prod(a.h, b);
-    return {p.h, __fmaf_rn(a.l, b, p.l)};
-}
-
 // acc += t; the low part collects the errors and is folded in at the end of an atom tile.
 __device__ __forceinline__ void df_acc(dfl &acc, dfl t) {
     const dfl s = two_sum(acc.h, t.h);

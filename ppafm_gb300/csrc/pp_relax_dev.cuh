@@ -72,13 +72,21 @@ __device__ __forceinline__ dfl spline_radial_df(const TipSpline &S, dfl x) {
 
 // ----------------------------------------------------------- interpolation
 
+// Force values at the corners of the cell that a stroke was in last, and the cell (-1: none).  A
+// probe stays in its cell for most iterations of a height, and the gathers, 32 lanes in 32
+// places, cost as much of the L1 as the arithmetic costs of the issue slots.
+struct Corners {
+    long long cell;
+    float x[8], y[8], z[8];
+};
+
 // Periodic trilinear interpolation of the force (Grid.h:93-111) at the grid coordinate
 // base + u (base integer, u double-float): float32 grid values, double-float weights and
 // compensated sums, so the only rounding left is that of the stored grid values.
 // NC: read-only (non-coherent) gathers; false for a grid written earlier in the same launch.
 template <bool NC = true>
 __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1, int n2, const int base[3],
-                                                const dfl u[3], dfl F[3]) {
+                                                const dfl u[3], dfl F[3], Corners &c) {
     auto ld = [&](const float4 *q) { return NC ? ldg4(q) : *q; };
     int ci[3];
     dfl t[3], m[3];
@@ -86,18 +94,25 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
     for (int k = 0; k < 3; k++) {
         t[k] = split_cell(u[k], ci[k]);
         ci[k] += base[k];
-        const dfl o = two_sum(1.f, -t[k].h);
+        const dfl o = fast_two_sum(1.f, -t[k].h);
         m[k] = {o.h, __fsub_rn(o.l, t[k].l)};
     }
     const int ix0 = wrap_index(ci[0], n0), iy0 = wrap_index(ci[1], n1), iz0 = wrap_index(ci[2], n2);
-    const int ix1 = (ix0 + 1 == n0) ? 0 : ix0 + 1;
-    const int iy1 = (iy0 + 1 == n1) ? 0 : iy0 + 1;
-    const int iz1 = (iz0 + 1 == n2) ? 0 : iz0 + 1;
-    const long long r00 = ((long long)ix0 * n1 + iy0) * n2, r01 = ((long long)ix0 * n1 + iy1) * n2;
-    const long long r10 = ((long long)ix1 * n1 + iy0) * n2, r11 = ((long long)ix1 * n1 + iy1) * n2;
-    // corner order (x, y, z bits): 000 001 010 011 100 101 110 111
-    const float4 c[8] = {ld(FE + r00 + iz0), ld(FE + r00 + iz1), ld(FE + r01 + iz0), ld(FE + r01 + iz1),
-                         ld(FE + r10 + iz0), ld(FE + r10 + iz1), ld(FE + r11 + iz0), ld(FE + r11 + iz1)};
+    const long long r00 = ((long long)ix0 * n1 + iy0) * n2;
+    if (r00 + iz0 != c.cell) {
+        c.cell = r00 + iz0;
+        const long long dx = ix0 + 1 == n0 ? -(long long)ix0 * n1 * n2 : (long long)n1 * n2;
+        const long long dy = iy0 + 1 == n1 ? -(long long)iy0 * n2 : (long long)n2;
+        const int dz = iz0 + 1 == n2 ? -iz0 : 1;
+        // corner order (x, y, z bits): 000 001 010 011 100 101 110 111
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float4 v = ld(FE + c.cell + ((k & 4) ? dx : 0) + ((k & 2) ? dy : 0) + ((k & 1) ? dz : 0));
+            c.x[k] = v.x;
+            c.y[k] = v.y;
+            c.z[k] = v.z;
+        }
+    }
     const dfl wxy[4] = {df_mul(m[0], m[1]), df_mul(m[0], t[1]), df_mul(t[0], m[1]), df_mul(t[0], t[1])};
     dfl w[8];
 #pragma unroll
@@ -110,7 +125,7 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
         dfl p[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const float v = comp == 0 ? c[k].x : (comp == 1 ? c[k].y : c[k].z);
+            const float v = comp == 0 ? c.x[k] : (comp == 1 ? c.y[k] : c.z[k]);
             p[k] = two_prod(w[k].h, v);
             p[k].l = __fmaf_rn(w[k].l, v, p[k].l);
         }
@@ -119,6 +134,14 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
         const dfl r = df_add_raw(df_add_raw(a0, a1), df_add_raw(a2, a3));
         F[comp] = two_sum(r.h, r.l);
     }
+}
+// The same, gathering every time.
+template <bool NC = true>
+__device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1, int n2, const int base[3],
+                                                const dfl u[3], dfl F[3]) {
+    Corners c;
+    c.cell = -1;
+    interp_force_df<NC>(FE, n0, n1, n2, base, u, F, c);
 }
 
 // interp_force_df split over a group of TPS lanes (TPS in {1, 2, 4, 8}, groups aligned in the
@@ -129,9 +152,9 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
 // result bit for bit.
 template <int TPS, bool NC = true>
 __device__ __forceinline__ void interp_force_df_group(const float4 *FE, int n0, int n1, int n2, const int base[3],
-                                                      const dfl u[3], dfl F[3], int sub, unsigned mask) {
+                                                      const dfl u[3], dfl F[3], int sub, unsigned mask, Corners &corners) {
     if constexpr (TPS == 1) {
-        interp_force_df<NC>(FE, n0, n1, n2, base, u, F);
+        interp_force_df<NC>(FE, n0, n1, n2, base, u, F, corners);
     } else {
         constexpr int CPL = 8 / TPS;  // corners per lane
         auto ld = [&](const float4 *q) { return NC ? ldg4(q) : *q; };
@@ -141,7 +164,7 @@ __device__ __forceinline__ void interp_force_df_group(const float4 *FE, int n0, 
         for (int k = 0; k < 3; k++) {
             t[k] = split_cell(u[k], ci[k]);
             ci[k] += base[k];
-            const dfl o = two_sum(1.f, -t[k].h);
+            const dfl o = fast_two_sum(1.f, -t[k].h);
             m[k] = {o.h, __fsub_rn(o.l, t[k].l)};
         }
         const int ix0 = wrap_index(ci[0], n0), iy0 = wrap_index(ci[1], n1), iz0 = wrap_index(ci[2], n2);

@@ -167,12 +167,13 @@ def tip_spline(spline):
 
 def autotune_relax_tps(ff, prm, xs, ys, zs, candidates=(1, 2, 4, 8), reps=2, apply=True):
     """Times relax_scan with each number of lanes per stroke on this scan and (apply) keeps the
-    fastest for the relaxations that follow.  Returns (best, {tps: ms})."""
+    fastest for the relaxations that follow.  1 stands for the library's default, which on small
+    scans has a lane for each axis of a stroke.  Returns (best, {tps: ms})."""
     times = {}
     out = {}
     try:
         for t in candidates:
-            check(lib().ppgpu_set_relax_tps(int(t)))
+            check(lib().ppgpu_set_relax_tps(0 if int(t) == 1 else int(t)))
             relax_scan(ff, prm, xs, ys, zs, out=out)  # warm-up (and buffers)
             torch.cuda.synchronize()
             a = torch.cuda.Event(enable_timing=True)
@@ -185,7 +186,7 @@ def autotune_relax_tps(ff, prm, xs, ys, zs, candidates=(1, 2, 4, 8), reps=2, app
             times[int(t)] = a.elapsed_time(b) / reps
     finally:
         best = min(times, key=times.get) if times else 1
-        check(lib().ppgpu_set_relax_tps(best if apply else 0))
+        check(lib().ppgpu_set_relax_tps(best if apply and best != 1 else 0))
     return best, times
 
 
