@@ -205,6 +205,14 @@ int ppgpu_fft_density_power(void *handle, float *rho, double B, int fix_negative
  * zero mean.  No counterpart in the reference (it reads potentials from DFT files). */
 int ppgpu_fft_poisson(void *handle, const float *rho_charge, const double *lvec, float *V, void *stream);
 
+/* The density-overlap force field (cli/conv_rho.py:24-88 + HighLevel.py:390-411) in one round
+ * trip of the plan's transforms: FE = scale_p P2F(rho_s^B, rho_t^B) + scale_e P2F(V, rho_t) with V
+ * the Hartree potential of rho_q (NULL: no electrostatics), energies included; P2F, the
+ * pre-processing (fix_negative, B) and V as in the three calls above.  Orthogonal cells only. */
+int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
+                             int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
+                             void *stream);
+
 /* AFMulator Hartree route, cross-correlation (FFTCrossCorrelation.correlate,
  * ppafm/ocl/field.py:800-840): E = IFFT(conj(FFT(rho)) FFT(V)) * scale / N on the plan's grid
  * (scale: the tip density's voxel volume in the reference).  The plan keeps the spectrum of

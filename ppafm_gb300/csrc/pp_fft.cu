@@ -254,6 +254,33 @@ __global__ void density_power_kernel(float *rho, long long N, const double *sums
     }
 }
 
+// A density for the overlap route in one pass: out = (v < 0 ? 0 : v)^B (fix_negative) or v^B, and
+// the sums whose ratio rescales the clipped density (density_sums_kernel).  The scale, a constant
+// factor of the spectrum, is left to overlap_spectra_kernel, so the density is read once.
+__global__ void overlap_density_kernel(const float *__restrict__ in, float *__restrict__ out, long long N, int fix_negative,
+                                       float B, double *sums) {
+    float s = 0.f, sc = 0.f, sp = 0.f, spc = 0.f;
+    auto add = [](float &acc, float &c, float v) {
+        const float t = acc + v;
+        c += (fabsf(acc) >= fabsf(v)) ? (acc - t) + v : (v - t) + acc;
+        acc = t;
+    };
+    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N; p += (long long)gridDim.x * blockDim.x) {
+        float v = in[p];
+        if (fix_negative) {
+            add(s, sc, v);
+            add(sp, spc, v > 0.f ? v : 0.f);
+            v = v < 0.f ? 0.f : v;
+        }
+        if (B != 1.f) v = powf(v, B);
+        out[p] = v;
+    }
+    if (!fix_negative) return;
+    block_sum_to((double)s + (double)sc, sums);
+    __syncthreads();
+    block_sum_to((double)sp + (double)spc, sums + 1);
+}
+
 // ------------------------------------------------------------------ Poisson
 
 struct PoissonPrm {
@@ -290,6 +317,63 @@ __global__ void poisson_kernel(C *Rk, PoissonPrm P) {
     const R sc = (sizeof(R) == 4) ? (R)P.sf : (R)P.s;
     const R f = (q == 0) ? (R)0 : sc / g2;
     Rk[q] = Cx<C>::make(r.x * f, r.y * f);
+}
+
+// ------------------------------------------------------------------ density overlap
+
+struct OverlapPrm {
+    SpecPrm sp;
+    PoissonPrm po;       // s, sf: 4 pi k_e, without 1/N (the potential is not transformed back)
+    double a, q;         // factors of the Pauli and the electrostatic spectra
+    int fix_negative, has_q;
+    float B;
+    const double *sums;  // [4] sums of rho_s, then of rho_t (fix_negative)
+};
+
+// The output spectra of the whole density-overlap force field from the four transformed densities:
+// C = a FFT(rho_s^B) conj(FFT(rho_t^B)) + q V conj(FFT(rho_t)), V = 4 pi k_e FFT(rho_q) / G^2, and
+// from C the energy and force spectra as in spectra_kernel.  W, T may be the first two of S4: each
+// thread reads its element of every input before it writes that element.
+template <typename C>
+__global__ void overlap_spectra_kernel(const C *W, const C *T, const C *__restrict__ Qk, const C *__restrict__ Rk, C *S4, OverlapPrm P) {
+    using R = typename Cx<C>::real;
+    __shared__ R s_fac;
+    if (threadIdx.x == 0) {
+        R f = (R)P.a;
+        if (P.fix_negative) {
+            const float fs = (float)(P.sums[0] / P.sums[1]), ft = (float)(P.sums[2] / P.sums[3]);
+            f *= (R)(P.B != 1.f ? powf(fs, P.B) : fs) * (R)(P.B != 1.f ? powf(ft, P.B) : ft);
+        }
+        s_fac = f;
+    }
+    __syncthreads();
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= P.sp.Nh) return;
+    const long long row = e / P.sp.nh2;
+    const int k = (int)(e - row * P.sp.nh2);
+    const int i = (int)(row / P.sp.n1), j = (int)(row - (long long)i * P.sp.n1);
+    const C w = W[e], t = T[e];
+    R cr = (w.x * t.x + w.y * t.y) * s_fac;
+    R ci = (w.y * t.x - w.x * t.y) * s_fac;
+    if (P.has_q) {
+        const R m0 = (R)freq(i, P.po.n0), m1 = (R)freq(j, P.po.n1), m2 = (R)freq(k, P.po.n2);
+        const R gx = m0 * pois_b<R>(P.po, 0) + m1 * pois_b<R>(P.po, 3) + m2 * pois_b<R>(P.po, 6);
+        const R gy = m0 * pois_b<R>(P.po, 1) + m1 * pois_b<R>(P.po, 4) + m2 * pois_b<R>(P.po, 7);
+        const R gz = m0 * pois_b<R>(P.po, 2) + m1 * pois_b<R>(P.po, 5) + m2 * pois_b<R>(P.po, 8);
+        const R sc = (sizeof(R) == 4) ? (R)P.po.sf : (R)P.po.s;
+        const R v = (e == 0) ? (R)0 : sc / (gx * gx + gy * gy + gz * gz) * (R)P.q;
+        const C q = Qk[e], r = Rk[e];
+        cr += v * (q.x * r.x + q.y * r.y);
+        ci += v * (q.y * r.x - q.x * r.y);
+    }
+    const R xo = (R)0.5 * (R)rolled_odd2(i, P.sp.n0), yo = (R)0.5 * (R)rolled_odd2(j, P.sp.n1), zo = (R)0.5 * (R)rolled_odd2(k, P.sp.n2);
+    const R sE = spec_s<R>(P.sp, false), sF = spec_s<R>(P.sp, true);
+    S4[e] = Cx<C>::make(cr * sE, ci * sE);
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++) {
+        const R zeta = (spec_z<R>(P.sp, 3 * ax) * xo + spec_z<R>(P.sp, 3 * ax + 1) * yo + spec_z<R>(P.sp, 3 * ax + 2) * zo) * sF;
+        S4[(ax + 1) * P.sp.Nh + e] = Cx<C>::make(zeta * ci, -zeta * cr);
+    }
 }
 
 // ------------------------------------------------------------ cross-correlation
@@ -431,6 +515,49 @@ extern "C" int ppgpu_fft_destroy(void *handle) {
     return set_ok();
 }
 
+// Coefficients of the output spectra (potential2forces_mem).
+static SpecPrm spec_params(const FFTPlan *P, const double *lvec) {
+    double L[9], dd[3], Li[9], det;
+    basis(P->n, lvec, L, dd);
+    inv3(L, Li, &det);  // LmatInv
+    const double detLinv = fabs(1.0 / det);
+    SpecPrm sp;
+    sp.n0 = P->n[0];
+    sp.n1 = P->n[1];
+    sp.n2 = P->n[2];
+    sp.nh2 = P->n[2] / 2 + 1;
+    for (int a = 0; a < 3; a++)
+        for (int j = 0; j < 3; j++) sp.z[3 * a + j] = Li[3 * a + j] / (P->n[j] * dd[j] * dd[j]) * dd[j];
+    const double dV = dd[0] * dd[1] * dd[2];
+    sp.sE = dV / detLinv / (double)P->N;
+    sp.sF = 2 * M_PI * dV / detLinv / (double)P->N;
+    sp.Nh = P->Nh;
+    for (int a = 0; a < 9; a++) sp.zf[a] = (float)sp.z[a];
+    sp.sEf = (float)sp.sE;
+    sp.sFf = (float)sp.sF;
+    return sp;
+}
+
+// Coefficients of the Poisson solve: reciprocal basis (rows of inv(cell)^T times 2 pi); false for a
+// singular cell.  s: 4 pi k_e times `norm`.
+static bool poisson_params(const FFTPlan *P, const double *lvec, double norm, PoissonPrm *pp) {
+    double cell[9], ci[9], det;
+    for (int k = 0; k < 9; k++) cell[k] = lvec[3 + k];
+    inv3(cell, ci, &det);
+    if (!(det != 0.0)) return false;
+    pp->n0 = P->n[0];
+    pp->n1 = P->n[1];
+    pp->n2 = P->n[2];
+    pp->nh2 = P->n[2] / 2 + 1;
+    for (int r = 0; r < 3; r++)
+        for (int c = 0; c < 3; c++) pp->b[3 * r + c] = 2 * M_PI * ci[3 * c + r];
+    pp->s = 4 * M_PI * 14.399645 * norm;
+    pp->Nh = P->Nh;
+    for (int a = 0; a < 9; a++) pp->bf[a] = (float)pp->b[a];
+    pp->sf = (float)pp->s;
+    return true;
+}
+
 // Forward transform of a float32 real grid into the spectrum buffer `out` (float64 plans
 // widen the grid into `stage` first).
 static int forward(FFTPlan *P, const float *x, void *out, double *stage, cudaStream_t st, const char *what) {
@@ -455,24 +582,7 @@ extern "C" int ppgpu_fft_potential2forces(void *handle, const float *V, const fl
     int rc;
     if ((rc = forward(P, V, P->Vk, stage, st, "forward V")) != PPGPU_OK) return rc;
     if ((rc = forward(P, rho, P->Rk, stage, st, "forward rho")) != PPGPU_OK) return rc;
-    double L[9], dd[3], Li[9], det;
-    basis(P->n, lvec, L, dd);
-    inv3(L, Li, &det);  // LmatInv
-    const double detLinv = fabs(1.0 / det);
-    SpecPrm sp;
-    sp.n0 = P->n[0];
-    sp.n1 = P->n[1];
-    sp.n2 = P->n[2];
-    sp.nh2 = P->n[2] / 2 + 1;
-    for (int a = 0; a < 3; a++)
-        for (int j = 0; j < 3; j++) sp.z[3 * a + j] = Li[3 * a + j] / (P->n[j] * dd[j] * dd[j]) * dd[j];
-    const double dV = dd[0] * dd[1] * dd[2];
-    sp.sE = dV / detLinv / (double)P->N;
-    sp.sF = 2 * M_PI * dV / detLinv / (double)P->N;
-    sp.Nh = P->Nh;
-    for (int a = 0; a < 9; a++) sp.zf[a] = (float)sp.z[a];
-    sp.sEf = (float)sp.sE;
-    sp.sFf = (float)sp.sF;
+    const SpecPrm sp = spec_params(P, lvec);
     const int with_e = (flags & PPGPU_FF_WITH_E) ? 1 : 0, acc = (flags & PPGPU_FF_ACCUMULATE) ? 1 : 0;
     if (P->f64) {
         spectra_kernel<cufftDoubleComplex><<<spec_blocks(P), FFT_THREADS, 0, st>>>(
@@ -545,22 +655,8 @@ extern "C" int ppgpu_fft_poisson(void *handle, const float *rho_charge, const do
     double *stage = (double *)P->planar;
     int rc;
     if ((rc = forward(P, rho_charge, P->Rk, stage, st, "forward rho")) != PPGPU_OK) return rc;
-    // reciprocal basis: rows of inv(cell)^T times 2 pi
-    double cell[9], ci[9], det;
-    for (int k = 0; k < 9; k++) cell[k] = lvec[3 + k];
-    inv3(cell, ci, &det);
-    if (!(det != 0.0)) return set_error(PPGPU_ERR_ARG, "poisson: singular cell");
     PoissonPrm pp;
-    pp.n0 = P->n[0];
-    pp.n1 = P->n[1];
-    pp.n2 = P->n[2];
-    pp.nh2 = P->n[2] / 2 + 1;
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++) pp.b[3 * r + c] = 2 * M_PI * ci[3 * c + r];
-    pp.s = 4 * M_PI * 14.399645 / (double)P->N;
-    pp.Nh = P->Nh;
-    for (int a = 0; a < 9; a++) pp.bf[a] = (float)pp.b[a];
-    pp.sf = (float)pp.s;
+    if (!poisson_params(P, lvec, 1.0 / (double)P->N, &pp)) return set_error(PPGPU_ERR_ARG, "poisson: singular cell");
     if (P->f64) {
         poisson_kernel<cufftDoubleComplex><<<spec_blocks(P), FFT_THREADS, 0, st>>>((cufftDoubleComplex *)P->Rk, pp);
         PPGPU_CHECK_LAUNCH("poisson_kernel");
@@ -572,6 +668,72 @@ extern "C" int ppgpu_fft_poisson(void *handle, const float *rho_charge, const do
         PPGPU_CHECK_LAUNCH("poisson_kernel");
         PPGPU_CUFFT(cufftExecC2R(P->c2r1, (cufftComplex *)P->Rk, (cufftReal *)V), "inverse V");
     }
+    return set_ok();
+}
+
+/* The density-overlap force field in one round trip: FE = scale_p P2F(rho_s^B, rho_t^B) +
+ * scale_e P2F(V, rho_t), V the Hartree potential of rho_q (NULL: no electrostatics), energies
+ * included, P2F as ppgpu_fft_potential2forces and the densities pre-processed as
+ * ppgpu_fft_density_power.  Both parts meet in the spectrum and the potential never leaves it: four
+ * transforms forward, four back, where the calls one by one take six and nine (256^3: 1.68 -> 0.93
+ * ms, bound by the passes of cuFFT's transforms over memory).  Orthogonal cells. */
+extern "C" int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
+                                        int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
+                                        void *stream) {
+    FFTPlan *P = (FFTPlan *)handle;
+    if (!P || !rho_s || !rho_t || !lvec || !FE) return set_error(PPGPU_ERR_ARG, "overlap_forces: null argument");
+    if (lvec[4] != 0.0 || lvec[5] != 0.0 || lvec[6] != 0.0 || lvec[8] != 0.0 || lvec[9] != 0.0 || lvec[10] != 0.0)
+        return set_error(PPGPU_ERR_ARG, "overlap_forces: the cell must be orthogonal");
+    cudaStream_t st = (cudaStream_t)stream;
+    OverlapPrm op;
+    op.sp = spec_params(P, lvec);
+    if (!poisson_params(P, lvec, 1.0, &op.po)) return set_error(PPGPU_ERR_ARG, "overlap_forces: singular cell");
+    op.a = scale_p;
+    op.q = scale_e;
+    op.fix_negative = fix_negative ? 1 : 0;
+    op.has_q = rho_q ? 1 : 0;
+    op.B = (float)B;
+    op.sums = P->sums;
+    PPGPU_CUFFT(cufftSetStream(P->r2c, st), "cufftSetStream");
+    PPGPU_CUFFT(cufftSetStream(P->c2r4, st), "cufftSetStream");
+    // the real planes are free until the inverse transform: the widened input of a float64 plan,
+    // then the pre-processed density
+    double *stage = (double *)P->planar;
+    float *work = P->f64 ? (float *)(stage + P->N) : (float *)P->planar;
+    const size_t cs = P->f64 ? sizeof(cufftDoubleComplex) : sizeof(cufftComplex);
+    void *Wk = P->S4, *Tk = (char *)P->S4 + P->Nh * cs;
+    const bool pre = fix_negative || B != 1.0;
+    if (fix_negative) PPGPU_CUDA(cudaMemsetAsync(P->sums, 0, 4 * sizeof(double), st), "clear sums");
+    int rc;
+    for (int d = 0; d < 2; d++) {
+        const float *src = d ? rho_t : rho_s;
+        if (pre) {
+            overlap_density_kernel<<<blocks_for(P->N), FFT_THREADS, 0, st>>>(src, work, P->N, op.fix_negative, op.B, P->sums + 2 * d);
+            PPGPU_CHECK_LAUNCH("overlap_density_kernel");
+            src = work;
+        }
+        if ((rc = forward(P, src, d ? Tk : Wk, stage, st, "forward density")) != PPGPU_OK) return rc;
+    }
+    if (rho_q) {
+        if ((rc = forward(P, rho_q, P->Vk, stage, st, "forward rho_q")) != PPGPU_OK) return rc;
+        if ((rc = forward(P, rho_t, P->Rk, stage, st, "forward rho_t")) != PPGPU_OK) return rc;
+    }
+    if (P->f64) {
+        overlap_spectra_kernel<cufftDoubleComplex><<<spec_blocks(P), FFT_THREADS, 0, st>>>(
+            (const cufftDoubleComplex *)Wk, (const cufftDoubleComplex *)Tk, (const cufftDoubleComplex *)P->Vk,
+            (const cufftDoubleComplex *)P->Rk, (cufftDoubleComplex *)P->S4, op);
+        PPGPU_CHECK_LAUNCH("overlap_spectra_kernel");
+        PPGPU_CUFFT(cufftExecZ2D(P->c2r4, (cufftDoubleComplex *)P->S4, (double *)P->planar), "inverse x4");
+        pack_fe_kernel<double><<<blocks_for(P->N), FFT_THREADS, 0, st>>>((float4 *)FE, (const double *)P->planar, P->N, 1.0, 1, 0);
+    } else {
+        overlap_spectra_kernel<cufftComplex><<<spec_blocks(P), FFT_THREADS, 0, st>>>(
+            (const cufftComplex *)Wk, (const cufftComplex *)Tk, (const cufftComplex *)P->Vk, (const cufftComplex *)P->Rk,
+            (cufftComplex *)P->S4, op);
+        PPGPU_CHECK_LAUNCH("overlap_spectra_kernel");
+        PPGPU_CUFFT(cufftExecC2R(P->c2r4, (cufftComplex *)P->S4, (cufftReal *)P->planar), "inverse x4");
+        pack_fe_kernel<float><<<blocks_for(P->N), FFT_THREADS, 0, st>>>((float4 *)FE, (const float *)P->planar, P->N, 1.0, 1, 0);
+    }
+    PPGPU_CHECK_LAUNCH("pack_fe_kernel");
     return set_ok();
 }
 
