@@ -3,12 +3,12 @@
 // Computes, for every grid point p, sums over atoms of the Lennard-Jones and
 // point-charge Coulomb interactions of the reference core:
 //   addAtomLJ      (ppafm/cpp/Forces.h:120-132)
-//   addAtomCoulomb (Forces.h:237-244) and the pz / dz2 finite-difference tips
-//                  (ppafm/cpp/ProbeParticle.cpp:192-209)
+//   addAtomCoulomb (Forces.h:237-244); the pz / dz2 tips are in pp_ff_tip.cu
 //   evalLJC_QZs_noPos (ppafm/ocl/cl/FF.cl:366-423) for the AFMulator grid
 // on the grid of GridShape (ppafm/cpp/Grid.h:29-36, 142-170).
 //
-// Design (GB300):
+// Pair by pair; grids of many boxes and atoms go to pp_ff_box.cu (launch_ff_box), which sums the
+// far atoms on interpolation nodes and the near ones as here.  Design (GB300):
 //  * Atom records (48 B: hi/lo split coordinates, charge, LJ coefficients) are streamed
 //    through shared memory in tiles of FF_TILE atoms by 1-D TMA bulk copies
 //    (cp.async.bulk + mbarrier, two stages), so the tile for step t+1 lands while
@@ -32,7 +32,6 @@
 #include <vector>
 
 #include "pp_common.cuh"
-#include "pp_df.cuh"
 #include "pp_ff_dev.cuh"
 
 namespace ppgpu {
@@ -200,168 +199,6 @@ static int ff64_dispatch(const FFParams &prm, int mode, int kind, cudaStream_t s
     }
 }
 
-// ------------------------------------------------- pz and dz2 tips in double-float
-//
-// getCoulombFF's finite-difference tips (ProbeParticle.cpp:192-209): the Coulomb field of the
-// same charge at heights dz - h, dz and dz + h (h = 0.1 A) with weights (-1, 0, 1)/h for pz and
-// (1, -2, 1)/h^2 for dz2.  The differences cancel (r/h)^2 of the significand, so they are formed
-// in double-float (pp_df.cuh, ~46 bits after the reciprocal root), as are the sums over the
-// atoms: what is left is the rounding of the stored float32, as in float64.  Float64 itself
-// issues at 1/64 of the float32 rate here, which made these tips 400 times an s tip.
-//
-// Bound by float32 instructions (~170 a pair for dz2, no memory traffic to speak of): a thread
-// owns TIP_P z points of one column, so the in-plane distance of an atom is formed once for all
-// of them, and TIP_P = 4 keeps their sums (6 or 8 registers a point) in registers at 4 CTAs a SM.
-// 342 charges on 200^3 points, dz2: 423 ms in float64, 16.7 ms here (19.4 with the energy); pz: 316 and 13.8 ms.
-
-constexpr int TIP_P = 4;
-constexpr int TIP_THREADS = 128;
-
-// acc += t; the low part collects the errors and is folded in at the end of an atom tile.
-__device__ __forceinline__ void df_acc(dfl &acc, dfl t) {
-    const dfl s = two_sum(acc.h, t.h);
-    acc.h = s.h;
-    acc.l = __fadd_rn(acc.l, __fadd_rn(s.l, t.l));
-}
-
-// 1/r and 1/r^3 of r^2: the approximate root y, then the series of (1 - e)^(-1/2) in its exact
-// residual e = 1 - r^2 y^2 (|e| < 2^-20, so two terms).
-struct InvR {
-    dfl i1, i3;
-};
-__device__ __forceinline__ InvR inv_r(dfl r2) {
-    const float y = rsqrt_approx(r2.h);
-    const dfl y2 = two_prod(y, y);
-    const dfl p = two_prod(r2.h, y2.h);
-    float e = __fsub_rn(__fsub_rn(1.f, p.h), p.l);
-    e = __fmaf_rn(-r2.h, y2.l, e);
-    e = __fmaf_rn(-r2.l, y2.h, e);
-    const float d = __fmul_rn(e, __fmaf_rn(0.375f, e, 0.5f));  // 1/r = y (1 + d)
-    const dfl y3 = two_prod(y, y2.h);
-    InvR o;
-    o.i1 = {y, __fmul_rn(y, d)};
-    // (1 + d)^3 = 1 + 3 d (1 + d) + d^3, the cube below 2^-60
-    o.i3 = {y3.h, __fmaf_rn(y3.h, __fmul_rn(3.f, __fmaf_rn(d, d, d)), __fmaf_rn(y, y2.l, y3.l))};
-    return o;
-}
-
-template <int KIND, bool WITH_E, bool ORTHO>
-__global__ void __launch_bounds__(TIP_THREADS, 4) ff_tip_kernel(const FFParams prm) {
-    static_assert(KIND == 1 || KIND == 2, "pz or dz2");
-    __shared__ __align__(16) float4 s_at[FF_TILE * FF_REC];
-    const int tid = threadIdx.x;
-    const long long chunk = (long long)blockIdx.x * TIP_THREADS + tid;
-    const bool valid = chunk < prm.nchunks;
-    int la = 0, lb = 0, lz0 = 0;
-    if (valid) {
-        const long long col = chunk / prm.nzc;
-        lz0 = (int)(chunk - col * prm.nzc) * TIP_P;
-        la = (int)(col / prm.ns[1]);
-        lb = (int)(col - (long long)la * prm.ns[1]);
-    }
-    const double ga = prm.i0[0] + la, gb = prm.i0[1] + lb, gc = prm.i0[2] + lz0;
-    constexpr int NXY = ORTHO ? 1 : TIP_P;  // in-plane positions of a thread's points
-    dfl px[NXY], py[NXY], pz[TIP_P];
-#pragma unroll
-    for (int i = 0; i < TIP_P; i++) {
-        if (i < NXY) {
-            px[i] = df_from(((prm.dA[0] * ga) + prm.dB[0] * gb) + prm.dC[0] * (gc + i));
-            py[i] = df_from(((prm.dA[1] * ga) + prm.dB[1] * gb) + prm.dC[1] * (gc + i));
-        }
-        pz[i] = df_from(((prm.dA[2] * ga) + prm.dB[2] * gb) + prm.dC[2] * (gc + i));
-    }
-    const dfl h = df_from(0.1), h2 = df_from(2 * 0.1), hh = df_from(0.1 * 0.1), eps = df_from(1.0e-8);
-    dfl F[3][TIP_P], A[TIP_P], E[TIP_P];  // A: the axial part of the z force, before its factor h
-#pragma unroll
-    for (int i = 0; i < TIP_P; i++) F[0][i] = F[1][i] = F[2][i] = A[i] = E[i] = {0.f, 0.f};
-
-    for (int base = 0; base < prm.ncharged; base += FF_TILE) {
-        const int nj = min(FF_TILE, prm.ncharged - base);
-        __syncthreads();
-        for (int i = tid; i < nj * FF_REC; i += TIP_THREADS) s_at[i] = prm.atoms[(size_t)base * FF_REC + i];
-        __syncthreads();
-        for (int j = 0; j < nj; j++) {
-            const float4 r0 = s_at[3 * j], r1 = s_at[3 * j + 1];  // negated coordinates
-            const float q = s_at[3 * j + 2].z;
-            dfl dx, dy, s, shh;
-#pragma unroll
-            for (int i = 0; i < TIP_P; i++) {
-                if (i < NXY) {
-                    dx = df_add(px[i], {r0.x, r0.z});
-                    dy = df_add(py[i], {r0.y, r0.w});
-                    s = df_add(df_add(df_sq(dx), df_sq(dy)), eps);
-                    shh = df_add(s, hh);
-                }
-                const dfl dz = df_add(pz[i], {r1.x, r1.y}), zz = df_sq(dz);
-                const dfl a = df_add(shh, zz), b = df_mul_raw(dz, h2);  // r^2 + h^2, 2 h dz
-                const InvR up = inv_r(df_add(a, b)), dn = inv_r(df_add(a, df_neg(b)));
-                const dfl D = df_add_raw(up.i3, df_neg(dn.i3)), S = df_add_raw(up.i3, dn.i3);
-                dfl rad, e;  // the field is q (rad (dx, dy, dz) + h ax z), ax = S (pz) or D (dz2)
-                if (KIND == 1) {
-                    rad = D;
-                    if (WITH_E) e = df_add_raw(up.i1, df_neg(dn.i1));
-                } else {
-                    const InvR md = inv_r(df_add(s, zz));
-                    rad = df_add_raw(S, {-2.f * md.i3.h, -2.f * md.i3.l});
-                    if (WITH_E) e = df_add_raw(df_add_raw(up.i1, dn.i1), {-2.f * md.i1.h, -2.f * md.i1.l});
-                }
-                rad = df_mul_raw(rad, q);
-                df_acc(F[0][i], df_mul_raw(rad, dx));
-                df_acc(F[1][i], df_mul_raw(rad, dy));
-                df_acc(F[2][i], df_mul_raw(rad, dz));
-                df_acc(A[i], df_mul_raw(KIND == 1 ? S : D, q));
-                if (WITH_E) df_acc(E[i], df_mul_raw(e, q));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < TIP_P; i++) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) F[k][i] = two_sum(F[k][i].h, F[k][i].l);
-            A[i] = two_sum(A[i].h, A[i].l);
-            if (WITH_E) E[i] = two_sum(E[i].h, E[i].l);
-        }
-    }
-    if (!valid) return;
-    const float w = KIND == 1 ? 10.f : 100.f;
-    float4 *out = prm.FE + ((long long)la * prm.ns[1] + lb) * prm.ns[2] + lz0;
-#pragma unroll
-    for (int i = 0; i < TIP_P; i++) {
-        if (lz0 + i >= prm.ns[2]) break;
-        float4 o;
-        o.x = df_round(df_mul_raw(F[0][i], w));
-        o.y = df_round(df_mul_raw(F[1][i], w));
-        o.z = df_round(df_mul_raw(df_add(F[2][i], df_mul_raw(A[i], h)), w));
-        o.w = WITH_E ? df_round(df_mul_raw(E[i], w)) : 0.f;
-        if (prm.accumulate) {
-            const float4 old = out[i];
-            o.x += old.x;
-            o.y += old.y;
-            o.z += old.z;
-            o.w += old.w;
-        }
-        out[i] = o;
-    }
-}
-
-template <int KIND>
-static int launch_ff_tip(FFParams &prm, bool with_e, bool ortho, cudaStream_t st) {
-    prm.nzc = (prm.ns[2] + TIP_P - 1) / TIP_P;
-    prm.nchunks = (long long)prm.ns[0] * prm.ns[1] * prm.nzc;
-    const long long nblk = (prm.nchunks + TIP_THREADS - 1) / TIP_THREADS;
-    if (nblk <= 0) return set_ok();
-    if (nblk > 0x7fffffffLL) return set_error(PPGPU_ERR_ARG, "ff grid too large (%lld blocks)", nblk);
-    const unsigned g = (unsigned)nblk;
-    if (with_e) {
-        if (ortho) ff_tip_kernel<KIND, true, true><<<g, TIP_THREADS, 0, st>>>(prm);
-        else ff_tip_kernel<KIND, true, false><<<g, TIP_THREADS, 0, st>>>(prm);
-    } else {
-        if (ortho) ff_tip_kernel<KIND, false, true><<<g, TIP_THREADS, 0, st>>>(prm);
-        else ff_tip_kernel<KIND, false, false><<<g, TIP_THREADS, 0, st>>>(prm);
-    }
-    PPGPU_CHECK_LAUNCH("ff_tip_kernel launch");
-    return set_ok();
-}
-
 // ------------------------------------------------------------------------ host
 
 // Threads per CTA of the single-grid kernel (ppgpu_set_ff_block): 0 = the default, 128.  At
@@ -420,8 +257,7 @@ static int ff_dispatch(FFParams &prm, int mode, int kind, bool with_e, bool orth
             return launch_ff_e<M_LJ, 4>(prm, with_e, ortho, st);
         case PPGPU_FF_COULOMB:
             if (kind == 0) return launch_ff_e<M_COUL, 4>(prm, with_e, ortho, st);
-            if (kind == 1) return launch_ff_tip<1>(prm, with_e, ortho, st);
-            if (kind == 2) return launch_ff_tip<2>(prm, with_e, ortho, st);
+            if (kind == 1 || kind == 2) return launch_ff_tip(prm, kind, with_e, ortho, st);
             return set_error(PPGPU_ERR_ARG, "coulomb kind %d not in {0,1,2}", kind);
         case PPGPU_FF_LJC:
             if (prm.ncharged <= SPLIT_MAX_CHARGED && !prm.accumulate)

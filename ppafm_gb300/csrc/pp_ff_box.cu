@@ -29,176 +29,12 @@
 #include <cmath>
 #include <cstring>
 
-#include "pp_common.cuh"
-#include "pp_df.cuh"
-#include "pp_ff_dev.cuh"
+#include "pp_ff_box_dev.cuh"
 
 namespace ppgpu {
 
-constexpr int BOX_N = 8;         // nodes per axis
-constexpr int BOX_N3 = 512;
-constexpr int BOX_S = 16;        // points per axis of a leaf, at most
-constexpr int BOX_NT = 256;      // threads of a leaf's CTA: 64 node columns x 4 quarters of the atoms
-constexpr int BOX_LEVELS = 3;    // levels above the leaves, at most
-constexpr int BOX_STAGE = 2 * BOX_NT;   // near atoms staged at a time (the space of a leaf's atom tiles)
-constexpr int BOX_NEAR = 2048;          // near atoms listed, as 16-bit indices (half of it as 32-bit ones)
 constexpr int BOX_FOLD = 64;     // near atoms summed before they join a point's running sum
 constexpr int BOX_P2 = 4;        // pairs of a thread's run of 8 nodes or points along z
-constexpr double BOX_KAPPA = 7.0;
-
-struct BoxPrm {
-    int s[3];    // leaf size in points (the last box of an axis may be smaller)
-    int nb[3];   // leaves per axis
-    int level;   // of this launch: 0 = leaves
-    int levels;  // levels above the leaves
-    float far2[BOX_LEVELS + 1];   // (7 H)^2, with the tip charges' offsets added to 7 H
-    float rep[BOX_LEVELS + 1];    // bound on 12 c12 / (6 c6 r^14), see box_far
-    dfl step[3][3];               // rows: grid steps along the axes
-    // Offsets of a run's points (every second point of a column) from its middle: a part of few
-    // bits, which a displacement's high part takes exactly, and the rest.
-    float offh[3][8], offl[3][8];
-};
-
-// ---------------------------------------------------------------- interpolation tables
-
-// Chebyshev nodes cos((2k + 1) pi / 16).
-struct ChebNodes {
-    double t[BOX_N] = {0.98078528040323044913, 0.83146961230254523708, 0.55557023301960222474, 0.19509032201612826785,
-                       -0.19509032201612826785, -0.55557023301960222474, -0.83146961230254523708, -0.98078528040323044913};
-    double w[BOX_N] = {};  // 1 / prod_{j != k} (t_k - t_j)
-    constexpr ChebNodes() {
-        for (int k = 0; k < BOX_N; k++) {
-            double p = 1.0;
-            for (int j = 0; j < BOX_N; j++)
-                if (j != k) p *= t[k] - t[j];
-            w[k] = 1.0 / p;
-        }
-    }
-};
-
-// Weights [points of the axis][point][node] of evenly spaced points over [-1, 1].
-struct ChebPoints {
-    float w[BOX_S + 1][BOX_S][BOX_N] = {};
-    constexpr ChebPoints() {
-        constexpr ChebNodes c;
-        for (int m = 1; m <= BOX_S; m++)
-            for (int i = 0; i < m; i++)
-                for (int k = 0; k < BOX_N; k++) {
-                    const double x = m > 1 ? (2.0 * i - (m - 1)) / (m - 1) : 0.0;
-                    double p = c.w[k];
-                    for (int j = 0; j < BOX_N; j++)
-                        if (j != k) p *= x - c.t[j];
-                    w[m][i][k] = (float)p;
-                }
-    }
-};
-__device__ const ChebPoints c_cheb_points = ChebPoints();
-
-// The nodes and their weights as double-floats.
-struct ChebNodesDf {
-    float th[BOX_N] = {}, tl[BOX_N] = {}, wh[BOX_N] = {}, wl[BOX_N] = {};
-    constexpr ChebNodesDf() {
-        constexpr ChebNodes c;
-        for (int k = 0; k < BOX_N; k++) {
-            th[k] = (float)c.t[k];
-            tl[k] = (float)(c.t[k] - (double)th[k]);
-            wh[k] = (float)c.w[k];
-            wl[k] = (float)(c.w[k] - (double)wh[k]);
-        }
-    }
-};
-__constant__ ChebNodesDf c_cheb = ChebNodesDf();
-__device__ __forceinline__ dfl cheb_t(int k) { return {c_cheb.th[k], c_cheb.tl[k]}; }
-
-// Lagrange basis polynomial k at x.
-__device__ __forceinline__ float cheb_basis(int k, dfl x) {
-    dfl p = {c_cheb.wh[k], c_cheb.wl[k]};
-#pragma unroll 1
-    for (int j = 0; j < BOX_N; j++)
-        if (j != k) p = df_mul(p, df_add(x, df_neg(cheb_t(j))));
-    return df_round(p);
-}
-
-// -------------------------------------------------------------------------- geometry
-
-// First and last point of box b of an axis at a level.
-__device__ __forceinline__ void box_span(const FFParams &prm, const BoxPrm &B, int level, int axis, int b, int &lo, int &hi) {
-    lo = (b << level) * B.s[axis];
-    hi = min(prm.ns[axis], ((b + 1) << level) * B.s[axis]) - 1;
-}
-
-// Half extent in grid steps, exact in float32 (a one-point box gets half a step; its weights are
-// those of x = 0).
-__device__ __forceinline__ float box_half(int lo, int hi) { return hi > lo ? 0.5f * (float)(hi - lo) : 0.5f; }
-
-__device__ __forceinline__ bool box_there(const BoxPrm &B, int level, const int b[3]) {
-    return b[0] <= (B.nb[0] - 1) >> level && b[1] <= (B.nb[1] - 1) >> level && b[2] <= (B.nb[2] - 1) >> level;
-}
-
-// What a box is handed from the level above lies in the points of its first leaf, in memory that
-// is the box's own until it has read it: first the slots of the interpolated sums, one for each
-// level, then each level's list of the atoms that no ancestor sums (their number, -1 for too many,
-// then 16-bit indices).  Both ends compute from the sizes alone what there is room for.
-struct BoxShare {
-    float4 *FE;         // first point
-    int m1, m2;         // points of the leaf along y, z
-    long long d0, d1;   // points of the grid from one x, y to the next
-    int pts, slots, room;  // points; those of the slots; those of one level's list (0: no list)
-};
-template <int NC>
-__device__ __forceinline__ BoxShare box_share(const FFParams &prm, const BoxPrm &B, int level, const int b[3]) {
-    int lo[3], m[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        int hi;
-        box_span(prm, B, 0, k, b[k] << level, lo[k], hi);
-        m[k] = hi - lo[k] + 1;
-    }
-    BoxShare s;
-    s.d1 = prm.ns[2];
-    s.d0 = (long long)prm.ns[1] * prm.ns[2];
-    s.FE = prm.FE + lo[0] * s.d0 + lo[1] * s.d1 + lo[2];
-    s.m1 = m[1];
-    s.m2 = m[2];
-    s.pts = m[0] * m[1] * m[2];
-    s.slots = B.levels * (NC * BOX_N3 / 4);
-    s.room = prm.natoms <= 65536 && s.pts > s.slots ? (s.pts - s.slots) / B.levels : 0;
-    return s;
-}
-__device__ __forceinline__ float4 *share_cell(const BoxShare &s, int e) {
-    const int col = e / s.m2, z = e - col * s.m2, x = col / s.m1, y = col - x * s.m1;
-    return s.FE + x * s.d0 + y * s.d1 + z;
-}
-template <int NC>
-__device__ __forceinline__ bool share_has_slot(const BoxShare &s, int level) {
-    return s.pts >= (level + 1) * (NC * BOX_N3 / 4);
-}
-template <int NC>
-__device__ __forceinline__ float4 *share_slot(const BoxShare &s, int level, int e) {
-    return share_cell(s, level * (NC * BOX_N3 / 4) + e);
-}
-__device__ __forceinline__ int *share_count(const BoxShare &s, int level) {
-    return reinterpret_cast<int *>(share_cell(s, s.slots + level * s.room));
-}
-__device__ __forceinline__ int share_list_size(const BoxShare &s) { return 8 * s.room - 2; }
-__device__ __forceinline__ unsigned short *share_list(const BoxShare &s, int level, int i) {
-    const int e = i + 2;  // behind the number
-    return reinterpret_cast<unsigned short *>(share_cell(s, s.slots + level * s.room + (e >> 3))) + (e & 7);
-}
-
-// Whether an atom (negated coordinates in r0, r1) is far from the box of centre c: explicitly
-// rounded operations, because the CTAs of several levels have to agree on it.  rep holds
-// 33 (7 H)^8: the interpolation error of the r^-13 force is 5e-6 of the term at 7 H and falls
-// with (7 H / r)^8, and 33 is its ratio to the 1.5e-7 allowed of the r^-7 force.
-template <int MODE>
-__device__ __forceinline__ bool box_far(const float4 &r0, const float4 &r1, const float4 &c, float far2, float rep) {
-    const float dx = __fadd_rn(c.x, r0.x), dy = __fadd_rn(c.y, r0.y), dz = __fadd_rn(c.z, r1.x);
-    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-    if (!(r2 >= far2)) return false;
-    if (MODE == M_COUL) return true;
-    const float r4 = __fmul_rn(r2, r2), r6 = __fmul_rn(r4, r2);
-    return __fmul_rn(fabsf(r1.w), rep) <= __fmul_rn(fabsf(r1.z), __fmul_rn(__fmul_rn(r6, r6), r2));
-}
 
 // --------------------------------------------------------------------------- sums
 
@@ -320,7 +156,7 @@ constexpr size_t box_smem() {
 template <int MODE, bool WITH_E, bool ORTHO, bool LEAF, int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_constant__ FFParams prm, const __grid_constant__ BoxPrm B) {
     static_assert(!LEAF || NT == BOX_NT, "the leaves' tables are laid out for 256 threads");
-    constexpr int WARPS = NT / 32, SUBS = NT / 64;
+    constexpr int SUBS = NT / 64;
     using Sums = BoxSums<MODE, WITH_E>;
     constexpr int NC = Sums::NC;
     // tiles: two atom tiles, then the nodes' sums, then the near atoms.  part: each thread's
@@ -331,9 +167,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
     __shared__ uint64_t bar[2];
     __shared__ unsigned short s_near[LEAF ? BOX_NEAR : 1];
     __shared__ unsigned short s_left[NT];  // upper boxes: a tile's atoms for the children
-    __shared__ unsigned char s_mid[NT];
-    __shared__ int s_cnt[2][WARPS];
-    __shared__ float4 s_centre[BOX_LEVELS + 1];  // this box (0) and its ancestors
+    __shared__ BoxPick<NT> pk;
     __shared__ dfl s_node[3][BOX_N][3];          // node positions: the parts along each axis (z: the middle only)
     __shared__ dfl s_pt[3][BOX_S][3];            // the points', runs along z from their middle (LEAF)
     __shared__ float s_off[3][8];                // offsets of the nodes along z
@@ -344,16 +178,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
     const int nat = (MODE == M_COUL) ? prm.ncharged : prm.natoms;
     const int ntiles = (nat + NT - 1) / NT;
     int b[3], lo[3], hi[3];
-    {
-        int r = blockIdx.x;
-        const int n2 = ((B.nb[2] - 1) >> level) + 1, n1 = ((B.nb[1] - 1) >> level) + 1;
-        b[2] = r % n2;
-        r /= n2;
-        b[1] = r % n1;
-        b[0] = r / n1;
-#pragma unroll
-        for (int k = 0; k < 3; k++) box_span(prm, B, level, k, b[k], lo[k], hi[k]);
-    }
+    box_of_cta(prm, B, level, b, lo, hi);
     BoxShare share;
     bool handed = false;  // the parent's sums are there
     int nlist = -1;       // atoms that the parent left to this box (-1: no list)
@@ -379,21 +204,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
             for (int t = 0; t < 2 && t < ntiles; t++) fetch(t);
     }
     // ---- tables of this box
-    if (warp == 1 && lane <= nanc) {
-        float c[3] = {0.f, 0.f, 0.f};
-        dfl s[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            int l, h;
-            box_span(prm, B, level + lane, a, b[a] >> lane, l, h);
-            const float g = 0.5f * (float)(l + h) + (float)prm.i0[a];
-#pragma unroll
-            for (int k = 0; k < 3; k++) s[k] = df_add(s[k], df_mul_f(B.step[a][k], g));
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) c[k] = df_round(s[k]);
-        s_centre[lane] = make_float4(c[0], c[1], c[2], 0.f);
-    }
+    if (warp == 1 && lane <= nanc) pk.centre[lane] = box_centre(prm, B, level, b, lane);
     if (warp == 0 && lane < 24) {  // (middle + half t_i) steps
         const int a = lane >> 3, i = lane & 7;
         int l, h;
@@ -422,15 +233,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
     } else {  // the children's nodes in this box: child c of an axis, its node pt & 7
         for (int i = tid; i < 3 * BOX_S * BOX_N; i += NT) {
             const int a = i / (BOX_S * BOX_N), pt = (i / BOX_N) % BOX_S, k = i % BOX_N;
-            const int ba = a == 0 ? b[0] : (a == 1 ? b[1] : b[2]), c = 2 * ba + (pt >> 3);
-            float w = 0.f;
-            if (c <= (B.nb[a] - 1) >> (level - 1)) {
-                int l, h, pl, ph;
-                box_span(prm, B, level - 1, a, c, l, h);
-                box_span(prm, B, level, a, ba, pl, ph);
-                const dfl x = df_add(df_mul_f(cheb_t(pt & 7), box_half(l, h)), {0.5f * (float)(l + h - pl - ph), 0.f});
-                w = cheb_basis(k, df_div(x, {box_half(pl, ph), 0.f}));
-            }
+            const float w = df_round(box_child_weight(prm, B, level, a, a == 0 ? b[0] : (a == 1 ? b[1] : b[2]), pt, k));
             if (a == 0) s_wx[pt][k] = w;
             if (a == 1) s_wy[pt][k] = w;
             if (a == 2) s_wz[pt >> 3][k][pt & 7] = w;
@@ -451,39 +254,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
     const bool wide = nat > 65536;  // near indices as int
     const int near_cap = wide ? BOX_NEAR / 2 : BOX_NEAR;
     auto near_at = [&](int i) -> int { return wide ? reinterpret_cast<const int *>(s_near)[i] : (int)s_near[i]; };
-    // Classifies the atoms of tile T, one a thread.  0: near (LEAF: summed at the points; else left
-    // to the children), 1: far, on this machine's nodes, 2: an ancestor's.  Lists those of class `want`
-    // in s_mid (nmid); place: where this thread's atom comes among those of class 0 (-1: not one).
     int nmid = 0, nzero = 0, place = -1;
-    auto pick = [&](const float4 *T, int nj, int want, bool ok) -> bool {
-        int c = 2;
-        if (ok && tid < nj) {
-            const float4 r0 = T[3 * tid], r1 = T[3 * tid + 1];
-            c = box_far<MODE>(r0, r1, s_centre[0], B.far2[level], B.rep[level]) ? 1 : 0;
-            for (int m = nanc; m > 0; m--)
-                if (box_far<MODE>(r0, r1, s_centre[m], B.far2[level + m], B.rep[level + m])) c = 2;
-        }
-        const unsigned bm = __ballot_sync(0xffffffffu, c == want), bz = __ballot_sync(0xffffffffu, c == 0);
-        if (lane == 0) {
-            s_cnt[0][warp] = __popc(bm);
-            s_cnt[1][warp] = __popc(bz);
-        }
-        if (__syncthreads_or(!ok)) return false;
-        const unsigned lt = (1u << lane) - 1u;
-        nmid = nzero = 0;
-        int m0 = 0, z0 = 0;
-#pragma unroll
-        for (int g = 0; g < WARPS; g++) {
-            if (g == warp) {
-                m0 = nmid;
-                z0 = nzero;
-            }
-            nmid += s_cnt[0][g];
-            nzero += s_cnt[1][g];
-        }
-        if (c == want) s_mid[m0 + __popc(bm & lt)] = (unsigned char)tid;
-        place = c == 0 ? z0 + __popc(bz & lt) : -1;
-        return true;
+    auto pick = [&](const float4 *T, int nj, int want, bool ok) {
+        return box_pick<MODE, NT>(B, pk, level, nanc, T, nj, want, ok, nmid, nzero, place);
     };
     // This thread's atom of tile t of the parent's list, or (all) of all atoms, into the tile.  The
     // list is gone once the box writes its points.
@@ -492,12 +265,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
         int j = -1;
         if (i < (all ? nat : ncand)) {
             j = all ? i : (int)*share_list(share, level, i);
-            const float4 *a = prm.atoms + (size_t)j * FF_REC;
-            float4 *T = tiles + ((t & 1) * NT + tid) * FF_REC;
-            const float4 c = ldg4(a + 2);
-            T[0] = ldg4(a);
-            T[1] = ldg4(a + 1);
-            T[2] = make_float4(c.x, c.y, c.z, j < prm.ncharged ? 1.f : 0.f);  // .w: charged
+            box_gather(prm, tiles + ((t & 1) * NT + tid) * FF_REC, j);
         }
         return j;
     };
@@ -530,19 +298,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
             }
         }
         __syncthreads();
-        if constexpr (!LEAF) {  // to the children's lists, a warp for a child
-#pragma unroll 1
-            for (int q = warp; q < 8; q += WARPS) {
-                const int ch[3] = {2 * b[0] + (q >> 2), 2 * b[1] + ((q >> 1) & 1), 2 * b[2] + (q & 1)};
-                if (!box_there(B, level - 1, ch)) continue;
-                const BoxShare cs = box_share<NC>(prm, B, level - 1, ch);
-                const int n = cs.room > 0 ? min(nzero, share_list_size(cs) - nnear) : 0;
-                for (int i = lane; i < n; i += 32) *share_list(cs, level - 1, nnear + i) = s_left[i];
-            }
-        }
+        if constexpr (!LEAF) box_leave<NC, NT>(prm, B, level, b, s_left, nzero, nnear);
         nnear += nzero;
         for (int i = sub; i < nmid; i += SUBS) {
-            const int j = s_mid[i];
+            const int j = pk.mid[i];
             const float4 r2r = T[3 * j + 2];
             const bool charged = nlist >= 0 ? r2r.w != 0.f : base + j < prm.ncharged;
             box_add<MODE, WITH_E, ORTHO, false>(prm, B, on, s_off, T[3 * j], T[3 * j + 1], r2r, charged, S);
@@ -560,15 +319,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
         __syncthreads();
         if (nlist < 0 && tid == 0 && t + 2 < ntiles) fetch(t + 2);
     }
-    if constexpr (!LEAF) {
-        if (tid < 8) {  // the number of the children's atoms
-            const int ch[3] = {2 * b[0] + (tid >> 2), 2 * b[1] + ((tid >> 1) & 1), 2 * b[2] + (tid & 1)};
-            if (box_there(B, level - 1, ch)) {
-                const BoxShare cs = box_share<NC>(prm, B, level - 1, ch);
-                if (cs.room > 0) *share_count(cs, level - 1) = nnear <= share_list_size(cs) ? nnear : -1;
-            }
-        }
-    }
+    if constexpr (!LEAF) box_leave_count<NC>(prm, B, level, b, nnear);
     __syncthreads();
     // ---- the nodes' sums: of all parts of the atoms and the parent's interpolated sums
     float4 *nodes = tiles;  // [NC][8][8][8]
@@ -713,7 +464,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ff_box_kernel(const __grid_const
                     pick(T, min(NT, nat - t * NT), 0, true);
                     __syncthreads();
                     for (int i = 0; i < nmid; i++) {
-                        const int j = s_mid[i];
+                        const int j = pk.mid[i];
                         const float4 r2r = T[3 * j + 2];
                         box_add<MODE, WITH_E, ORTHO, true>(prm, B, o, nullptr, T[3 * j], T[3 * j + 1], r2r, r2r.w != 0.f, S);
                     }
@@ -814,43 +565,11 @@ static int launch_box_mode(const FFParams &prm, const BoxPrm &B, bool with_e, bo
     return ortho ? launch_box<MODE, false, true>(prm, B, st) : launch_box<MODE, false, false>(prm, B, st);
 }
 
-// The leaves of a grid and the levels above them.
-static void box_plan(const FFParams &prm, BoxPrm *B, double *half0) {
-    memset(B, 0, sizeof(*B));
-    for (int k = 0; k < 3; k++) {
-        const int parts = (prm.ns[k] + BOX_S - 1) / BOX_S;
-        B->s[k] = (prm.ns[k] + parts - 1) / parts;
-        if (k == 2) B->s[k] = (B->s[k] + 1) / 2 * 2;  // two threads a column
-        B->nb[k] = (prm.ns[k] + B->s[k] - 1) / B->s[k];
-    }
-    const double *d[3] = {prm.dA, prm.dB, prm.dC};
-    for (int a = 0; a < 3; a++)
-        for (int k = 0; k < 3; k++) B->step[a][k] = df_from(d[a][k]);
-    for (int k = 0; k < 3; k++)
-        for (int i = 0; i < 8; i++) {
-            const double v = prm.dC[k] * (2 * i - 7);
-            const double h = rint(v * 8192.0) / 8192.0;  // multiples of 2^-13
-            B->offh[k][i] = (float)h;
-            B->offl[k][i] = (float)(v - (double)(float)h);
-        }
-    double qz = 0.0;  // tip charges beside the probe's position
-    for (int k = 0; k < prm.nqa; k++) qz = std::max(qz, (double)fabsf(prm.QZa[k]));
-    for (int l = 0; l <= BOX_LEVELS; l++) {
-        double H2 = 0.0;  // half diagonal of a whole box
-        for (int c = 0; c < 4; c++) {
-            double r2 = 0.0;
-            for (int k = 0; k < 3; k++) {
-                const double e0 = 0.5 * ((B->s[0] << l) - 1), e1 = 0.5 * ((B->s[1] << l) - 1), e2 = 0.5 * ((B->s[2] << l) - 1);
-                const double v = e0 * prm.dA[k] + (c & 1 ? -e1 : e1) * prm.dB[k] + (c & 2 ? -e2 : e2) * prm.dC[k];
-                r2 += v * v;
-            }
-            H2 = std::max(H2, r2);
-        }
-        const double H = sqrt(H2), R = BOX_KAPPA * H + qz;
-        if (l == 0) *half0 = H;
-        B->far2[l] = (float)(R * R);
-        B->rep[l] = (float)std::min(33.0 * pow(BOX_KAPPA * H, 8.0), 3e38);
-    }
+// Largest distance of a tip charge from the probe's position.
+static double tip_reach(const FFParams &prm) {
+    double q = 0.0;
+    for (int k = 0; k < prm.nqa; k++) q = std::max(q, (double)fabsf(prm.QZa[k]));
+    return q;
 }
 
 // Grids and atoms summed by boxes.  Measured on a GB300, ff_block -> boxes (LJ + Coulomb, all atoms
@@ -867,7 +586,7 @@ static void box_plan(const FFParams &prm, BoxPrm *B, double *half0) {
 bool ff_box_rule(const FFParams &prm, int mode, int *levels) {
     BoxPrm B;
     double H;
-    box_plan(prm, &B, &H);
+    box_plan(prm, BOX_KAPPA, tip_reach(prm), &B, &H);
     const double boxes = (double)B.nb[0] * B.nb[1] * B.nb[2];
     const double nat = mode == M_COUL ? prm.ncharged : prm.natoms;
     const double pairs = nat + (mode == M_QZS && prm.nqa > 0 ? 4.0 * prm.ncharged : 0.0);
@@ -881,7 +600,7 @@ bool ff_box_rule(const FFParams &prm, int mode, int *levels) {
 int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, int levels, cudaStream_t st) {
     BoxPrm B;
     double H;
-    box_plan(prm, &B, &H);
+    box_plan(prm, BOX_KAPPA, tip_reach(prm), &B, &H);
     B.levels = prm.accumulate ? 0 : std::min(levels, BOX_LEVELS);
     switch (mode) {
         case M_LJ:

@@ -49,3 +49,63 @@ def test_tip_field_matches_float64(gpulib, kind, cell, n2, natoms):
     whole = run(False, False)
     sub = ff.compute_subgrid(i0, ns, atoms, na, nch, D.FF_COULOMB, kind=kind, with_E=True).view(*ns, 4).cpu().numpy()
     assert (sub == whole[2:7, 3:10].astype(np.float32)).all()
+
+
+BOXES = [
+    # n, step, tilted, charges, spread in z, energy, accumulate
+    ((113, 97, 130), 0.1, False, 200, 0.3, True, False),
+    ((113, 97, 130), 0.1, True, 200, 0.3, False, False),
+    ((97, 113, 128), 0.07, False, 300, 0.3, False, True),
+    ((97, 113, 128), 0.07, True, 300, 0.3, True, True),
+    ((180, 177, 161), 0.1, False, 400, 0.3, True, False),  # a level above the leaves
+    ((180, 177, 161), 0.1, False, 400, 0.3, False, False),
+    ((113, 112, 97), 0.1, False, 3000, 8.0, False, False),  # more near charges than the list holds
+    ((113, 112, 97), 0.1, True, 900, 8.0, True, False),  # near charges staged in parts
+]
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("case", BOXES, ids=lambda c: "-".join(map(str, c)))
+def test_tip_boxes_match_float64(gpulib, kind, case):
+    """The same tips by boxes, on sub-boxes of the grid: as above, and 1e-9 of the pairs' own fields
+    (below 6 q / r^3 for pz, 20 q / r^4 for dz2) for the interpolation of the far ones."""
+    import torch
+
+    from ppafm_gb300 import device as D
+
+    n, step, tilted, natoms, dz, energy, accumulate = case
+    rng = np.random.default_rng(natoms + n[0])
+    cell = np.diag(np.array(n) * step)
+    if tilted:
+        cell[1, 0], cell[2, 0], cell[2, 1] = 0.7, -0.9, 0.5
+    L = np.diag(cell)
+    R = np.column_stack([rng.uniform(-0.7 * L[0], 1.7 * L[0], natoms), rng.uniform(-0.7 * L[1], 1.7 * L[1], natoms), rng.uniform(-dz, 0.3, natoms)])
+    if dz > 1:
+        R[:, :2] = L[:2] / 2 + rng.normal(0, 2.5, (natoms, 2))
+    q = rng.uniform(-0.3, 0.3, natoms) * 14.399645
+    atoms, na, nch = D.pack_atoms(R, None, q)
+    ff = D.DeviceFF(n, cell)
+    ff.FE.fill_(0.25 if accumulate else float("nan"))
+    got = ff.compute(atoms, na, nch, D.FF_COULOMB, kind=kind, with_E=energy, accumulate=accumulate).grid4.cpu().numpy().astype(np.float64)
+    assert np.isfinite(got).all()
+    ns = (5, 6, 9)
+    corners = [(0, 0, 0)] + [tuple(int(rng.integers(0, n[k] - ns[k] + 1)) for k in range(3)) for _ in range(8)] + [tuple(n[k] - ns[k] for k in range(3))]
+    w = 20.0 if kind == 1 else 400.0
+    for i0 in corners:
+        ref = ff.compute_subgrid(i0, ns, atoms, na, nch, D.FF_COULOMB, kind=kind, with_E=True, f64=True).view(-1, 4).cpu().numpy().astype(np.float64)
+        g = got[i0[0] : i0[0] + 5, i0[1] : i0[1] + 6, i0[2] : i0[2] + 9].reshape(-1, 4)
+        P = (np.indices(ns).reshape(3, -1).T + np.array(i0)) @ (cell / np.array(n)[:, None])
+        r = np.sqrt(np.maximum(((P[:, None] - R[None]) ** 2).sum(-1), 1e-8))
+        pair = 6 * np.abs(q) / r**3 if kind == 1 else 20 * np.abs(q) / r**4
+        floor = (w * np.abs(q) / r**2).sum(1) * 2.0**-42 + 1e-9 * pair.sum(1)
+        floor_E = (w * np.abs(q) / r).sum(1) * 2.0**-42 + 1e-9 * (pair * r).sum(1)
+        tol = 2.0**-23 * np.abs(ref) + np.column_stack([floor, floor, floor, floor_E])
+        if accumulate:
+            tol += 2.0**-23 * (np.abs(ref) + 0.25)
+            ref = ref + 0.25
+        k = 4 if energy else 3
+        d = np.abs(g - ref)
+        assert (d[:, :k] <= tol[:, :k]).all(), (i0, float((d[:, :k] / tol[:, :k]).max()))
+        if not energy:
+            assert (g[:, 3] == (0.25 if accumulate else 0.0)).all()
+    assert torch.isfinite(ff.FE).all()
