@@ -13,21 +13,21 @@
 
 namespace ppgpu {
 
-constexpr int BOX_N = 8;         // nodes per axis
-constexpr int BOX_N3 = 512;
+// N, below: nodes per axis, 8 or 10.
 constexpr int BOX_S = 16;        // points per axis of a leaf, at most
 constexpr int BOX_NT = 256;      // threads of a leaf's CTA
 constexpr int BOX_LEVELS = 3;    // levels above the leaves, at most
-constexpr int BOX_STAGE = 2 * BOX_NT;   // near atoms staged at a time (the space of a leaf's atom tiles)
-constexpr int BOX_NEAR = 2048;          // near atoms listed, as 16-bit indices (half of it as 32-bit ones)
-constexpr double BOX_KAPPA = 7.0;
+constexpr int BOX_STAGE = BOX_NT;       // near atoms staged at a time
+constexpr int BOX_LEFT = 4096;          // atoms that a CTA of an upper box leaves to the children
+constexpr int BOX_NEAR = 1024;          // near atoms listed, as 16-bit indices (half of it as 32-bit ones)
 
 struct BoxPrm {
-    int s[3];    // leaf size in points (the last box of an axis may be smaller)
+    int s[3];    // points of a leaf along an axis, one more for the first rem[axis] leaves; the last may have fewer
+    int rem[3];
     int nb[3];   // leaves per axis
     int level;   // of this launch: 0 = leaves
     int levels;  // levels above the leaves
-    float far2[BOX_LEVELS + 1];   // (7 H)^2, with the tip charges' offsets added to 7 H
+    float far2[BOX_LEVELS + 1];   // (kappa H)^2, with the tip charges' offsets added to kappa H
     float rep[BOX_LEVELS + 1];    // bound on 12 c12 / (6 c6 r^14), see box_far
     dfl step[3][3];               // rows: grid steps along the axes
     // Offsets of a run's points (every second point of a column) from its middle: a part of few
@@ -37,15 +37,22 @@ struct BoxPrm {
 
 // ---------------------------------------------------------------- interpolation tables
 
-// Chebyshev nodes cos((2k + 1) pi / 16).
+// Chebyshev nodes cos((2k + 1) pi / 2N).
+template <int N>
 struct ChebNodes {
-    double t[BOX_N] = {0.98078528040323044913, 0.83146961230254523708, 0.55557023301960222474, 0.19509032201612826785,
-                       -0.19509032201612826785, -0.55557023301960222474, -0.83146961230254523708, -0.98078528040323044913};
-    double w[BOX_N] = {};  // 1 / prod_{j != k} (t_k - t_j)
+    double t[N] = {}, w[N] = {};  // w: 1 / prod_{j != k} (t_k - t_j)
     constexpr ChebNodes() {
-        for (int k = 0; k < BOX_N; k++) {
+        constexpr double t8[4] = {0.98078528040323044913, 0.83146961230254523708, 0.55557023301960222474, 0.19509032201612826785};
+        constexpr double t10[5] = {0.98768834059513772619, 0.89100652418836786236, 0.70710678118654752440, 0.45399049973954679156,
+                                   0.15643446504023086901};
+        static_assert(N == 8 || N == 10, "nodes");
+        for (int k = 0; k < N / 2; k++) {
+            t[k] = N == 8 ? t8[k < 4 ? k : 3] : t10[k];
+            t[N - 1 - k] = -t[k];
+        }
+        for (int k = 0; k < N; k++) {
             double p = 1.0;
-            for (int j = 0; j < BOX_N; j++)
+            for (int j = 0; j < N; j++)
                 if (j != k) p *= t[k] - t[j];
             w[k] = 1.0 / p;
         }
@@ -53,30 +60,38 @@ struct ChebNodes {
 };
 
 // Weights [points of the axis][point][node] of evenly spaced points over [-1, 1].
+template <int N>
 struct ChebPoints {
-    float w[BOX_S + 1][BOX_S][BOX_N] = {}, l[BOX_S + 1][BOX_S][BOX_N] = {};  // high and low parts
+    float w[BOX_S + 1][BOX_S][N] = {}, l[BOX_S + 1][BOX_S][N] = {};  // high and low parts
     constexpr ChebPoints() {
-        constexpr ChebNodes c;
+        constexpr ChebNodes<N> c;
         for (int m = 1; m <= BOX_S; m++)
             for (int i = 0; i < m; i++)
-                for (int k = 0; k < BOX_N; k++) {
+                for (int k = 0; k < N; k++) {
                     const double x = m > 1 ? (2.0 * i - (m - 1)) / (m - 1) : 0.0;
                     double p = c.w[k];
-                    for (int j = 0; j < BOX_N; j++)
+                    for (int j = 0; j < N; j++)
                         if (j != k) p *= x - c.t[j];
                     w[m][i][k] = (float)p;
                     l[m][i][k] = (float)(p - (double)w[m][i][k]);
                 }
     }
 };
-static __device__ const ChebPoints c_cheb_points = ChebPoints();
+static __device__ const ChebPoints<8> c_points8 = ChebPoints<8>();
+static __device__ const ChebPoints<10> c_points10 = ChebPoints<10>();
+template <int N>
+__device__ __forceinline__ const ChebPoints<N> &cheb_points() {
+    if constexpr (N == 8) return c_points8;
+    else return c_points10;
+}
 
 // The nodes and their weights as double-floats.
+template <int N>
 struct ChebNodesDf {
-    float th[BOX_N] = {}, tl[BOX_N] = {}, wh[BOX_N] = {}, wl[BOX_N] = {};
+    float th[N] = {}, tl[N] = {}, wh[N] = {}, wl[N] = {};
     constexpr ChebNodesDf() {
-        constexpr ChebNodes c;
-        for (int k = 0; k < BOX_N; k++) {
+        constexpr ChebNodes<N> c;
+        for (int k = 0; k < N; k++) {
             th[k] = (float)c.t[k];
             tl[k] = (float)(c.t[k] - (double)th[k]);
             wh[k] = (float)c.w[k];
@@ -84,24 +99,43 @@ struct ChebNodesDf {
         }
     }
 };
-static __constant__ ChebNodesDf c_cheb = ChebNodesDf();
-__device__ __forceinline__ dfl cheb_t(int k) { return {c_cheb.th[k], c_cheb.tl[k]}; }
+static __constant__ ChebNodesDf<8> c_nodes8 = ChebNodesDf<8>();
+static __constant__ ChebNodesDf<10> c_nodes10 = ChebNodesDf<10>();
+template <int N>
+__device__ __forceinline__ const ChebNodesDf<N> &cheb_nodes() {
+    if constexpr (N == 8) return c_nodes8;
+    else return c_nodes10;
+}
+template <int N>
+__device__ __forceinline__ dfl cheb_t(int k) {
+    return {cheb_nodes<N>().th[k], cheb_nodes<N>().tl[k]};
+}
 
-// Lagrange basis polynomial k at x.
-__device__ __forceinline__ dfl cheb_basis(int k, dfl x) {
-    dfl p = {c_cheb.wh[k], c_cheb.wl[k]};
-#pragma unroll 1
-    for (int j = 0; j < BOX_N; j++)
-        if (j != k) p = df_mul(p, df_add(x, df_neg(cheb_t(j))));
-    return p;
+// The Lagrange basis polynomials at x, from the products of the factors before and behind each.
+template <int N, class Store>
+__device__ __forceinline__ void cheb_row(dfl x, Store store) {
+    dfl behind[N];
+    dfl p = {1.f, 0.f};
+#pragma unroll
+    for (int k = N - 1; k >= 0; k--) {
+        behind[k] = p;
+        p = df_mul(p, df_add(x, df_neg(cheb_t<N>(k))));
+    }
+    p = {1.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        store(k, df_mul(df_mul(p, behind[k]), {cheb_nodes<N>().wh[k], cheb_nodes<N>().wl[k]}));
+        p = df_mul(p, df_add(x, df_neg(cheb_t<N>(k))));
+    }
 }
 
 // -------------------------------------------------------------------------- geometry
 
 // First and last point of box b of an axis at a level.
 __device__ __forceinline__ void box_span(const FFParams &prm, const BoxPrm &B, int level, int axis, int b, int &lo, int &hi) {
-    lo = (b << level) * B.s[axis];
-    hi = min(prm.ns[axis], ((b + 1) << level) * B.s[axis]) - 1;
+    const int first = b << level, end = (b + 1) << level;
+    lo = first * B.s[axis] + min(first, B.rem[axis]);
+    hi = min(prm.ns[axis], end * B.s[axis] + min(end, B.rem[axis])) - 1;
 }
 
 // Half extent in grid steps, exact in float32 (a one-point box gets half a step; its weights are
@@ -113,16 +147,19 @@ __device__ __forceinline__ bool box_there(const BoxPrm &B, int level, const int 
 }
 
 // What a box is handed from the level above lies in the points of its first leaf, in memory that
-// is the box's own until it has read it: first the slots of the interpolated sums, one for each
-// level, then each level's list of the atoms that no ancestor sums (their number, -1 for too many,
-// then 16-bit indices).  Both ends compute from the sizes alone what there is room for.
+// is the box's own until it has read it: the interpolated sums, then the list of the atoms that no
+// ancestor sums (their number, -1 for too many, then 16-bit indices).  The box leaves the same to
+// its children, to the first one in the same place: it has read its sums by then, and the list
+// it writes runs behind the tiles that it has read.  Both ends compute from the sizes alone what
+// there is room for.
 struct BoxShare {
     float4 *FE;         // first point
     int m1, m2;         // points of the leaf along y, z
     long long d0, d1;   // points of the grid from one x, y to the next
-    int pts, slots, room;  // points; those of the slots; those of one level's list (0: no list)
+    int pts, room;      // points; those for the list (0: no list)
+    float r1, r2;       // 1 / m1, 1 / m2
 };
-template <int NC>
+template <int N, int NC>
 __device__ __forceinline__ BoxShare box_share(const FFParams &prm, const BoxPrm &B, int level, const int b[3]) {
     int lo[3], m[3];
 #pragma unroll
@@ -137,49 +174,51 @@ __device__ __forceinline__ BoxShare box_share(const FFParams &prm, const BoxPrm 
     s.FE = prm.FE + lo[0] * s.d0 + lo[1] * s.d1 + lo[2];
     s.m1 = m[1];
     s.m2 = m[2];
+    s.r1 = __fdiv_rn(1.f, (float)m[1]);
+    s.r2 = __fdiv_rn(1.f, (float)m[2]);
     s.pts = m[0] * m[1] * m[2];
-    s.slots = B.levels * (NC * BOX_N3 / 4);
-    s.room = prm.natoms <= 65536 && s.pts > s.slots ? (s.pts - s.slots) / B.levels : 0;
+    s.room = prm.natoms <= 65536 ? max(0, s.pts - NC * (N * N * N / 4)) : 0;
     return s;
 }
 __device__ __forceinline__ float4 *share_cell(const BoxShare &s, int e) {
-    const int col = e / s.m2, z = e - col * s.m2, x = col / s.m1, y = col - x * s.m1;
+    // quotients of numbers up to 4096 by 16 at most: the rounding stays far below the half added
+    const int col = (int)(((float)e + 0.5f) * s.r2), z = e - col * s.m2;
+    const int x = (int)(((float)col + 0.5f) * s.r1), y = col - x * s.m1;
     return s.FE + x * s.d0 + y * s.d1 + z;
 }
-template <int NC>
-__device__ __forceinline__ bool share_has_slot(const BoxShare &s, int level) {
-    return s.pts >= (level + 1) * (NC * BOX_N3 / 4);
+// Whether there is room for the sums: cells 0 to NC N^3 / 4 - 1, NC components of the nodes.
+template <int N, int NC>
+__device__ __forceinline__ bool share_has_sums(const BoxShare &s) {
+    return s.pts >= NC * (N * N * N / 4);
 }
-template <int NC>
-__device__ __forceinline__ float4 *share_slot(const BoxShare &s, int level, int e) {
-    return share_cell(s, level * (NC * BOX_N3 / 4) + e);
-}
-__device__ __forceinline__ int *share_count(const BoxShare &s, int level) {
-    return reinterpret_cast<int *>(share_cell(s, s.slots + level * s.room));
+template <int N, int NC>
+__device__ __forceinline__ int *share_count(const BoxShare &s) {
+    return reinterpret_cast<int *>(share_cell(s, NC * (N * N * N / 4)));
 }
 __device__ __forceinline__ int share_list_size(const BoxShare &s) { return 8 * s.room - 2; }
-__device__ __forceinline__ unsigned short *share_list(const BoxShare &s, int level, int i) {
+template <int N, int NC>
+__device__ __forceinline__ unsigned short *share_list(const BoxShare &s, int i) {
     const int e = i + 2;  // behind the number
-    return reinterpret_cast<unsigned short *>(share_cell(s, s.slots + level * s.room + (e >> 3))) + (e & 7);
+    return reinterpret_cast<unsigned short *>(share_cell(s, NC * (N * N * N / 4) + (e >> 3))) + (e & 7);
 }
 
 // Whether an atom (negated coordinates in r0, r1) is far from the box of centre c: explicitly
-// rounded operations, because the CTAs of several levels have to agree on it.  rep holds
-// 33 (7 H)^8: the interpolation error of the r^-13 force is 5e-6 of the term at 7 H and falls
-// with (7 H / r)^8, and 33 is its ratio to the 1.5e-7 allowed of the r^-7 force.
-template <int MODE>
+// rounded operations, because the CTAs of several levels have to agree on it.  rep: the interpolation
+// error of the r^-13 force at kappa H (5e-6 of the term with 8 nodes at 7, 2e-5 with 10 at 4.25) over
+// the 1.5e-7 allowed of the r^-7 force, times (kappa H)^N, with whose power over r it falls.
+template <int MODE, int N>
 __device__ __forceinline__ bool box_far(const float4 &r0, const float4 &r1, const float4 &c, float far2, float rep) {
     const float dx = __fadd_rn(c.x, r0.x), dy = __fadd_rn(c.y, r0.y), dz = __fadd_rn(c.z, r1.x);
     const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
     if (!(r2 >= far2)) return false;
     if (MODE == M_COUL) return true;
-    const float r4 = __fmul_rn(r2, r2), r6 = __fmul_rn(r4, r2);
-    return __fmul_rn(fabsf(r1.w), rep) <= __fmul_rn(fabsf(r1.z), __fmul_rn(__fmul_rn(r6, r6), r2));
+    const float r4 = __fmul_rn(r2, r2), r8 = __fmul_rn(r4, r4), rn = __fmul_rn(r8, N == 8 ? __fmul_rn(r4, r2) : r8);  // r^(6 + N)
+    return __fmul_rn(fabsf(r1.w), rep) <= __fmul_rn(fabsf(r1.z), fminf(rn, 3e38f));
 }
 
-// This CTA's box at a level and its points; boxes are numbered along z first.
-__device__ __forceinline__ void box_of_cta(const FFParams &prm, const BoxPrm &B, int level, int b[3], int lo[3], int hi[3]) {
-    int r = blockIdx.x;
+// A CTA's box at a level and its points; boxes are numbered along z first.
+__device__ __forceinline__ void box_of_cta(const FFParams &prm, const BoxPrm &B, int level, int box, int b[3], int lo[3], int hi[3]) {
+    int r = box;
     const int n2 = ((B.nb[2] - 1) >> level) + 1, n1 = ((B.nb[1] - 1) >> level) + 1;
     b[2] = r % n2;
     r /= n2;
@@ -203,15 +242,15 @@ __device__ __forceinline__ float4 box_centre(const FFParams &prm, const BoxPrm &
     return make_float4(df_round(s[0]), df_round(s[1]), df_round(s[2]), 0.f);
 }
 
-// Weight of node k of this box at node pt & 7 of its child pt >> 3 along an axis (0: no such child).
-__device__ __forceinline__ dfl box_child_weight(const FFParams &prm, const BoxPrm &B, int level, int a, int ba, int pt, int k) {
-    const int c = 2 * ba + (pt >> 3);
-    if (c > (B.nb[a] - 1) >> (level - 1)) return {0.f, 0.f};
+// Node i of child c (0 or 1) along an axis, in the box's own [-1, 1]; false: no such child.
+template <int N>
+__device__ __forceinline__ bool box_child_node(const FFParams &prm, const BoxPrm &B, int level, int a, int ba, int c, int i, dfl &x) {
+    if (2 * ba + c > (B.nb[a] - 1) >> (level - 1)) return false;
     int l, h, pl, ph;
-    box_span(prm, B, level - 1, a, c, l, h);
+    box_span(prm, B, level - 1, a, 2 * ba + c, l, h);
     box_span(prm, B, level, a, ba, pl, ph);
-    const dfl x = df_add(df_mul_f(cheb_t(pt & 7), box_half(l, h)), {0.5f * (float)(l + h - pl - ph), 0.f});
-    return cheb_basis(k, df_div(x, {box_half(pl, ph), 0.f}));
+    x = df_div(df_add(df_mul_f(cheb_t<N>(i), box_half(l, h)), {0.5f * (float)(l + h - pl - ph), 0.f}), {box_half(pl, ph), 0.f});
+    return true;
 }
 
 // What the threads of a CTA share while they go through the atoms.
@@ -227,16 +266,16 @@ struct BoxPick {
 // class `want` in S.mid (nmid of them); nzero: number of class 0; place: where this thread's atom
 // comes among those (-1: not one).  Threads must meet before they read S.mid.  False when a
 // thread's tile did not land.
-template <int MODE, int NT>
+template <int MODE, int N, int NT>
 __device__ __forceinline__ bool box_pick(const BoxPrm &B, BoxPick<NT> &S, int level, int nanc, const float4 *T, int nj, int want,
                                          bool ok, int &nmid, int &nzero, int &place) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int c = 2;
     if (ok && tid < nj) {
         const float4 r0 = T[3 * tid], r1 = T[3 * tid + 1];
-        c = box_far<MODE>(r0, r1, S.centre[0], B.far2[level], B.rep[level]) ? 1 : 0;
+        c = box_far<MODE, N>(r0, r1, S.centre[0], B.far2[level], B.rep[level]) ? 1 : 0;
         for (int m = nanc; m > 0; m--)
-            if (box_far<MODE>(r0, r1, S.centre[m], B.far2[level + m], B.rep[level + m])) c = 2;
+            if (box_far<MODE, N>(r0, r1, S.centre[m], B.far2[level + m], B.rep[level + m])) c = 2;
     }
     const unsigned bm = __ballot_sync(0xffffffffu, c == want), bz = __ballot_sync(0xffffffffu, c == 0);
     if (lane == 0) {
@@ -270,43 +309,84 @@ __device__ __forceinline__ void box_gather(const FFParams &prm, float4 *T, int j
     T[2] = make_float4(c.x, c.y, c.z, j < prm.ncharged ? 1.f : 0.f);
 }
 
-// A tile's atoms of class 0 (n of them, in `left`, after `before` others) to the children's lists, a
-// warp for a child.
-template <int NC, int NT>
+// The atoms that this CTA leaves to the children of its box (n of them, in `left`; none of them
+// when there are more), behind `before` others of `all`: their lists, and from one CTA the number.
+template <int N, int NC, int NT>
 __device__ __forceinline__ void box_leave(const FFParams &prm, const BoxPrm &B, int level, const int b[3], const unsigned short *left,
-                                          int n, int before) {
+                                          int n, int before, int all, bool number) {
+    if (all < 0) n = 0;
 #pragma unroll 1
     for (int q = threadIdx.x >> 5; q < 8; q += NT / 32) {
         const int ch[3] = {2 * b[0] + (q >> 2), 2 * b[1] + ((q >> 1) & 1), 2 * b[2] + (q & 1)};
         if (!box_there(B, level - 1, ch)) continue;
-        const BoxShare cs = box_share<NC>(prm, B, level - 1, ch);
-        const int m = cs.room > 0 ? min(n, share_list_size(cs) - before) : 0;
-        for (int i = threadIdx.x & 31; i < m; i += 32) *share_list(cs, level - 1, before + i) = left[i];
+        const BoxShare cs = box_share<N, NC>(prm, B, level - 1, ch);
+        if (cs.room == 0) continue;
+        const int m = min(n, share_list_size(cs) - before), lane = threadIdx.x & 31;
+        for (int i = lane; i < m; i += 32) *share_list<N, NC>(cs, before + i) = left[i];
+        if (number && lane == 0) *share_count<N, NC>(cs) = all <= share_list_size(cs) ? all : -1;
     }
 }
 
-// The number of the children's atoms in front of their lists.
-template <int NC>
-__device__ __forceinline__ void box_leave_count(const FFParams &prm, const BoxPrm &B, int level, const int b[3], int n) {
-    const int q = threadIdx.x;
-    if (q >= 8) return;
-    const int ch[3] = {2 * b[0] + (q >> 2), 2 * b[1] + ((q >> 1) & 1), 2 * b[2] + (q & 1)};
-    if (!box_there(B, level - 1, ch)) return;
-    const BoxShare cs = box_share<NC>(prm, B, level - 1, ch);
-    if (cs.room > 0) *share_count(cs, level - 1) = n <= share_list_size(cs) ? n : -1;
+// ----------------------------------------------------------------------- clusters
+//
+// An upper box may be worked on by the CTAs of a cluster: each takes a part of the atoms and some
+// of the children, and reads the others' sums of the nodes from their shared memory.
+
+__device__ __forceinline__ int cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+__device__ __forceinline__ int cluster_size() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return (int)r;
+}
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float4 cluster_ld4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ int cluster_ldi(uint32_t a) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void async_copy16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // ------------------------------------------------------------------------------ host
 
-// The leaves of a grid and the levels above them; half0: half diagonal of a leaf.  Far at a level:
-// kappa half diagonals, and the reach of the tip's charges.
-static inline void box_plan(const FFParams &prm, double kappa, double reach, BoxPrm *B, double *half0) {
+// The leaves of a grid and the levels above them; half0: H of a leaf.  Far at a level: kappa H, and
+// the reach of the tip's charges.  H is the half diagonal, or that of a cube of the longest
+// edge: the error follows the nearest singularity beside the longest edge, and kappa is a cube's.
+static inline void box_plan(const FFParams &prm, int N, double kappa, double reach, BoxPrm *B, double *half0) {
     memset(B, 0, sizeof(*B));
     for (int k = 0; k < 3; k++) {
-        const int parts = (prm.ns[k] + BOX_S - 1) / BOX_S;
-        B->s[k] = (prm.ns[k] + parts - 1) / parts;
+        B->nb[k] = (prm.ns[k] + BOX_S - 1) / BOX_S;
+        if (B->nb[k] == 0) continue;  // no points
+        B->s[k] = (prm.ns[k] + B->nb[k] - 1) / B->nb[k];
         if (k == 2) B->s[k] = (B->s[k] + 1) / 2 * 2;  // two threads a column
-        B->nb[k] = (prm.ns[k] + B->s[k] - 1) / B->s[k];
+        // Whole leaves and a smaller last one, unless that is too small to be handed sums.
+        if (prm.ns[k] - (B->nb[k] - 1) * B->s[k] < (N == 8 ? 8 : 12)) {
+            B->s[k] = prm.ns[k] / B->nb[k];
+            B->rem[k] = prm.ns[k] % B->nb[k];
+        }
     }
     const double *d[3] = {prm.dA, prm.dB, prm.dC};
     for (int a = 0; a < 3; a++)
@@ -319,21 +399,54 @@ static inline void box_plan(const FFParams &prm, double kappa, double reach, Box
             B->offl[k][i] = (float)(v - (double)(float)h);
         }
     for (int l = 0; l <= BOX_LEVELS; l++) {
-        double H2 = 0.0;  // half diagonal of a whole box
+        double e[3], H2 = 0.0;  // half extents of the largest box, in steps
+        for (int k = 0; k < 3; k++) e[k] = 0.5 * ((B->s[k] << l) + std::min(1 << l, B->rem[k]) - 1);
         for (int c = 0; c < 4; c++) {
             double r2 = 0.0;
             for (int k = 0; k < 3; k++) {
-                const double e0 = 0.5 * ((B->s[0] << l) - 1), e1 = 0.5 * ((B->s[1] << l) - 1), e2 = 0.5 * ((B->s[2] << l) - 1);
-                const double v = e0 * prm.dA[k] + (c & 1 ? -e1 : e1) * prm.dB[k] + (c & 2 ? -e2 : e2) * prm.dC[k];
+                const double v = e[0] * prm.dA[k] + (c & 1 ? -e[1] : e[1]) * prm.dB[k] + (c & 2 ? -e[2] : e[2]) * prm.dC[k];
                 r2 += v * v;
             }
             H2 = std::max(H2, r2);
         }
+        for (int a = 0; a < 3; a++) {
+            double r2 = 0.0;
+            for (int k = 0; k < 3; k++) r2 += e[a] * d[a][k] * e[a] * d[a][k];
+            H2 = std::max(H2, 3.0 * r2);
+        }
         const double H = sqrt(H2), R = kappa * H + reach;
         if (l == 0) *half0 = H;
         B->far2[l] = (float)(R * R);
-        B->rep[l] = (float)std::min(33.0 * pow(kappa * H, 8.0), 3e38);
+        B->rep[l] = (float)std::min((N == 8 ? 33.0 : 130.0) * pow(kappa * H, (double)N), 3e38);
     }
 }
+
+// CTAs of a cluster for each of n upper boxes: enough to fill the SMs (two CTAs each).
+static inline int box_cluster(long long n) {
+    int c = 1;
+    while (c < 8 && n * c < 456) c *= 2;
+    return c;
+}
+
+// A level above the leaves: n boxes, a cluster of CTAs each.
+template <class Kernel>
+static int launch_box_up(Kernel kernel, int smem, long long n, const FFParams &prm, const BoxPrm &B, cudaStream_t st) {
+    const int c = box_cluster(n);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(n * c));
+    cfg.blockDim = dim3(BOX_NT);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    PPGPU_CUDA(cudaLaunchKernelEx(&cfg, kernel, prm, B), "ff box launch");
+    return PPGPU_OK;
+}
+
+int launch_ff_box10(const FFParams &prm, const BoxPrm &B, int mode, bool with_e, bool ortho, cudaStream_t st);  // pp_ff_box10.cu
 
 }  // namespace ppgpu

@@ -49,10 +49,9 @@ inline void ff_set_offsets(FFParams &prm) {
         for (int i = 0; i < FF_MAX_P; i++) prm.off[c][i] = (float)(prm.dC[c] * i);
 }
 
-// Force fields by boxes (pp_ff_box.cu): whether a grid and its atoms are summed that way, with
-// how many levels of boxes above the leaves, and the launch.
-bool ff_box_rule(const FFParams &prm, int mode, int *levels);
-int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, int levels, cudaStream_t st);
+// Force fields by boxes (pp_ff_box.cu): whether a grid and its atoms are summed that way.
+bool ff_box_rule(const FFParams &prm, int mode, bool with_e);
+int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st);
 // The pz (1) and dz2 (2) Coulomb tips in double-float (pp_ff_tip.cu).
 int launch_ff_tip(FFParams &prm, int kind, bool with_e, bool ortho, cudaStream_t st);
 

@@ -8,7 +8,7 @@
 // issues at 1/64 of the float32 rate here, which made these tips 400 times an s tip.
 //
 // Bound by float32 instructions (~210 a pair for dz2, no memory traffic to speak of).
-//   342 charges on 200^3 points: dz2 423 ms in float64, 16.7 ms pair by pair here, 2.44 by boxes (error
+//   342 charges on 200^3 points: dz2 423 ms in float64, 16.7 ms pair by pair here, 1.86 by boxes (error
 //   against 64 bits 5.6e-8 in all three: the stored float32's rounding).
 #include "pp_ff_box_dev.cuh"
 
@@ -171,92 +171,219 @@ __global__ void __launch_bounds__(TIP_THREADS, 4) ff_tip_kernel(const FFParams p
 // ------------------------------------------------------------------------- by boxes
 //
 // The method of pp_ff_box.cu in double-float: the charges far from a box of up to 16^3 points
-// (R >= 9 H + h) are summed on 8^3 nodes, which with the smoother Coulomb terms leaves 6e-10 of a
+// (R >= 5 H + h) are summed on 10^3 nodes, which with the smoother Coulomb terms leaves 4e-10 of a
 // pair's field, a hundredth of the stored value's rounding; nodes, weights and sums are
-// double-floats.  256 threads: for the nodes 128 halves of a node column x 2 parts of the atoms,
-// for the points runs of every fourth point of a column (neighbours write neighbouring points).
-// The interpolation goes along x (line), then along y for half of the box's x at a time (plane),
-// then along z into a run's sums.  128 registers, two CTAs a SM.
+// double-floats.  256 threads: 250 with four of the nodes each; for the points runs of every fourth
+// point of a column (neighbours write neighbouring points).  The interpolation goes along x (line),
+// then along y for four of the box's x at a time (plane), then along z into a run's sums.  128
+// registers, two CTAs a SM.
 
-constexpr double TIP_KAPPA = 9.0;
+constexpr double TIP_KAPPA = 5.0;
 constexpr int TIP_NT = 256;
+constexpr int TIP_N = 10, TIP_N2 = 100, TIP_N3 = 1000;  // nodes
+constexpr int TIP_X = 4;  // of the box's x in the plane
 
 // acc += w v (both double-floats).
 __device__ __forceinline__ void df_fma(dfl &acc, dfl w, dfl v) { df_acc(acc, df_mul_raw(w, v)); }
 
-template <bool WITH_E>
-constexpr size_t tip_box_smem() {
-    return sizeof(float4) * 2 * TIP_NT * FF_REC + 2 * sizeof(dfl) * (WITH_E ? 4 : 3) * BOX_S * 64;
+// Parts of the nodes' positions along the axes.
+__device__ __forceinline__ void tip_node_table(const FFParams &prm, const BoxPrm &B, int level, const int b[3], int i, dfl (*node)[TIP_N][3]) {
+    const int a = i / TIP_N, n = i % TIP_N;
+    int l, h;
+    box_span(prm, B, level, a, a == 0 ? b[0] : (a == 1 ? b[1] : b[2]), l, h);
+    const dfl g = df_add(df_mul_f(cheb_t<TIP_N>(n), box_half(l, h)), {0.5f * (float)(l + h) + (float)prm.i0[a], 0.f});
+#pragma unroll
+    for (int k = 0; k < 3; k++) node[a][n][k] = df_mul(B.step[a][k], g);
 }
 
-template <int KIND, bool WITH_E, bool ORTHO, bool LEAF>
-__global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constant__ FFParams prm, const __grid_constant__ BoxPrm B) {
-    constexpr int K = WITH_E ? 4 : 3, NC = 2 * K, NT = TIP_NT;  // components; floats of a node
+// Positions of a thread's four nodes.
+__device__ __forceinline__ void tip_nodes(const dfl (*node)[TIP_N][3], int tid, dfl (*p)[TIP_P]) {
+#pragma unroll
+    for (int i = 0; i < TIP_P; i++) {
+        const int e = min(TIP_P * tid + i, TIP_N3 - 1), ia = e / TIP_N2, ib = e / TIP_N % TIP_N, ic = e % TIP_N;
+#pragma unroll
+        for (int k = 0; k < 3; k++) p[k][i] = df_add(df_add(node[0][ia][k], node[1][ib][k]), node[2][ic][k]);
+    }
+}
+
+// Upper boxes, as box_up_kernel: a cluster of CTAs a box, parts of the charges and of the children each.
+// Shared memory: an atom tile, then the sums along z; this CTA's sums, then those along y; the
+// box's sums.
+template <bool WITH_E>
+struct TipUpSmem {
+    static constexpr int K = WITH_E ? 4 : 3;
+    static constexpr size_t own = sizeof(dfl) * K * TIP_N3, sum = 2 * own, size = 3 * own;
+    static_assert(own >= sizeof(float4) * TIP_NT * FF_REC, "the tile's space");
+};
+
+template <int KIND, bool WITH_E>
+__global__ void __launch_bounds__(TIP_NT, 2) tip_up_kernel(const __grid_constant__ FFParams prm, const __grid_constant__ BoxPrm B) {
+    using Smem = TipUpSmem<WITH_E>;
+    constexpr int K = Smem::K, NC = 2 * K, NT = TIP_NT, C4 = K * TIP_N3 / 2;
     extern __shared__ __align__(128) unsigned char tip_raw[];
-    float4 *tiles = reinterpret_cast<float4 *>(tip_raw);                                   // atoms; the nodes' sums; near atoms
-    dfl *line = reinterpret_cast<dfl *>(tip_raw + sizeof(float4) * 2 * NT * FF_REC);      // [K][x][8][8]
-    dfl *plane = line + K * BOX_S * 64;                                                    // [K][8 of x][y][8]; parts of the nodes' sums
-    __shared__ unsigned short s_near[LEAF ? BOX_NEAR : 1];
-    __shared__ unsigned short s_left[NT];
+    float4 *tile = reinterpret_cast<float4 *>(tip_raw);
+    dfl *lz = reinterpret_cast<dfl *>(tip_raw), *own = reinterpret_cast<dfl *>(tip_raw + Smem::own), *sum = reinterpret_cast<dfl *>(tip_raw + Smem::sum);
+    __shared__ unsigned short s_left[BOX_LEFT];
+    __shared__ int s_count;
     __shared__ BoxPick<NT> pk;
-    __shared__ dfl s_node[3][BOX_N][3], s_pt[3][BOX_S][3];                // parts of the nodes' and the points' positions
-    __shared__ dfl s_wx[BOX_S][BOX_N], s_wy[BOX_S][BOX_N], s_wz[BOX_S][BOX_N];
+    __shared__ dfl s_node[3][TIP_N][3], s_w[3][2][TIP_N][TIP_N];  // weights: [axis][child][node of the box][node of the child]
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int level = LEAF ? 0 : B.level, nat = prm.ncharged;
+    const int level = B.level, rank = cluster_rank(), ncta = cluster_size(), nat = prm.ncharged;
     int b[3], lo[3], hi[3];
-    box_of_cta(prm, B, level, b, lo, hi);
+    box_of_cta(prm, B, level, blockIdx.x / ncta, b, lo, hi);
     BoxShare share;
     bool handed = false;
     int nlist = -1;
     if (level < B.levels) {
-        share = box_share<NC>(prm, B, level, b);
-        handed = share_has_slot<NC>(share, level);
-        if (handed && share.room > 0) nlist = *share_count(share, level);
+        share = box_share<TIP_N, NC>(prm, B, level, b);
+        handed = share_has_sums<TIP_N, NC>(share);
+        if (handed && share.room > 0) nlist = *share_count<TIP_N, NC>(share);
+    }
+    const int nanc = handed ? B.levels - level : 0;
+    const int ncand = nlist >= 0 ? nlist : nat, per = (ncand + ncta - 1) / ncta;
+    const int first = min(rank * per, ncand), last = min(first + per, ncand);
+    if (warp == 1 && lane <= nanc) pk.centre[lane] = box_centre(prm, B, level, b, lane);
+    if (warp == 0 && lane < 3 * TIP_N) tip_node_table(prm, B, level, b, lane, s_node);
+    if (tid >= 64 && tid < 64 + 6 * TIP_N) {
+        const int i = tid - 64, a = i / (2 * TIP_N), c = i / TIP_N % 2, n = i % TIP_N;
+        dfl x;
+        if (box_child_node<TIP_N>(prm, B, level, a, a == 0 ? b[0] : (a == 1 ? b[1] : b[2]), c, n, x))
+            cheb_row<TIP_N>(x, [&](int k, dfl w) { s_w[a][c][k][n] = w; });
+    }
+    __syncthreads();
+    const bool on_nodes = tid < TIP_N3 / TIP_P;
+    dfl p[3][TIP_P];
+    TipSums S;
+    S.zero();
+    tip_nodes(s_node, tid, p);
+    int nmid = 0, nzero = 0, place = -1, nleft = 0;
+    for (int i0 = first; i0 < last; i0 += NT) {
+        const int i = i0 + tid;
+        int j0 = -1;
+        if (i < last) {
+            j0 = nlist >= 0 ? (int)*share_list<TIP_N, NC>(share, i) : i;
+            box_gather(prm, tile + tid * FF_REC, j0);
+        }
+        box_pick<M_COUL, TIP_N, NT>(B, pk, level, nanc, tile, min(NT, last - i0), 1, true, nmid, nzero, place);
+        if (place >= 0 && nleft + place < BOX_LEFT) s_left[nleft + place] = (unsigned short)j0;
+        nleft += nzero;
+        __syncthreads();
+        for (int q = on_nodes ? 0 : nmid; q < nmid; q++) {
+            const int j = pk.mid[q];
+            tip_add<KIND, WITH_E, false>(p, tile[3 * j], tile[3 * j + 1], tile[3 * j + 2].z, S);
+        }
+        S.fold<WITH_E>();
+        __syncthreads();
+    }
+    if (on_nodes) {
+#pragma unroll
+        for (int k = 0; k < K; k++)
+#pragma unroll
+            for (int i = 0; i < TIP_P; i++) own[k * TIP_N3 + TIP_P * tid + i] = S.get(k, i);
+    }
+    if (tid == 0) s_count = prm.natoms <= 65536 && nleft <= BOX_LEFT ? nleft : -1;
+    cluster_meet();
+    int before = 0, all = 0;
+    for (int q = 0; q < ncta; q++) {
+        const int n = cluster_ldi(cluster_addr(&s_count, q));
+        if (q < rank) before += n;
+        all = n < 0 || all < 0 ? -1 : all + n;
+    }
+    for (int i = tid; i < C4; i += NT) {  // two nodes
+        float4 v = handed ? *share_cell(share, i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < ncta; q++) {
+            const float4 o = cluster_ld4(cluster_addr(reinterpret_cast<const float4 *>(own) + i, q));
+            const dfl s0 = df_add({v.x, v.y}, {o.x, o.y}), s1 = df_add({v.z, v.w}, {o.z, o.w});
+            v = make_float4(s0.h, s0.l, s1.h, s1.l);
+        }
+        reinterpret_cast<float4 *>(sum)[i] = v;
+    }
+    cluster_meet();
+    box_leave<TIP_N, NC, NT>(prm, B, level, b, s_left, nleft, before, all, rank == 0);
+    dfl *ly = own;
+    for (int q = rank; q < 8; q += ncta) {
+        const int c[3] = {q >> 2, (q >> 1) & 1, q & 1}, ch[3] = {2 * b[0] + c[0], 2 * b[1] + c[1], 2 * b[2] + c[2]};
+        if (!box_there(B, level - 1, ch)) continue;
+        const BoxShare cs = box_share<TIP_N, NC>(prm, B, level - 1, ch);
+        if (!share_has_sums<TIP_N, NC>(cs)) continue;
+        auto along = [&](const dfl *v, int step, int axis, int n) -> dfl {  // at the child's node n
+            dfl s = {0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < TIP_N; k++) df_fma(s, s_w[axis][c[axis]][k][n], v[k * step]);
+            return two_sum(s.h, s.l);
+        };
+        for (int i = tid; i < K * TIP_N3; i += NT) lz[i] = along(sum + i / TIP_N * TIP_N, 1, 2, i % TIP_N);
+        __syncthreads();
+        for (int i = tid; i < K * TIP_N3; i += NT) ly[i] = along(lz + i / TIP_N2 * TIP_N2 + i % TIP_N, TIP_N, 1, i / TIP_N % TIP_N);
+        __syncthreads();
+        for (int i = tid; i < C4; i += NT) {
+            const int k = i / (TIP_N3 / 2), r = i - k * (TIP_N3 / 2), x = r / (TIP_N2 / 2), yz = 2 * (r - x * (TIP_N2 / 2));
+            const dfl s0 = along(ly + k * TIP_N3 + yz, TIP_N2, 0, x), s1 = along(ly + k * TIP_N3 + yz + 1, TIP_N2, 0, x);
+            *share_cell(cs, i) = make_float4(s0.h, s0.l, s1.h, s1.l);
+        }
+        __syncthreads();
+    }
+}
+
+// Leaves.  Shared memory: two atom tiles or the nodes' sums (then near atoms), the line and the plane.
+template <bool WITH_E>
+struct TipSmem {
+    static constexpr int K = WITH_E ? 4 : 3, XS = BOX_S;
+    static constexpr size_t tiles = sizeof(float4) * 2 * TIP_NT * FF_REC, nodes = sizeof(dfl) * K * TIP_N3;
+    static constexpr size_t line = tiles > nodes ? tiles : nodes, plane = line + sizeof(dfl) * K * XS * TIP_N2;
+    static constexpr size_t size = plane + sizeof(dfl) * K * TIP_X * XS * TIP_N;
+};
+
+template <int KIND, bool WITH_E, bool ORTHO>
+__global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constant__ FFParams prm, const __grid_constant__ BoxPrm B) {
+    using Smem = TipSmem<WITH_E>;
+    constexpr int K = Smem::K, NC = 2 * K, NT = TIP_NT, XS = Smem::XS, level = 0;  // NC: floats of a node
+    extern __shared__ __align__(128) unsigned char tip_raw[];
+    float4 *tiles = reinterpret_cast<float4 *>(tip_raw);
+    dfl *line = reinterpret_cast<dfl *>(tip_raw + Smem::line);    // [K][x][10][10]
+    dfl *plane = reinterpret_cast<dfl *>(tip_raw + Smem::plane);  // [K][x - xh][y][10]
+    __shared__ unsigned short s_near[BOX_NEAR];
+    __shared__ BoxPick<NT> pk;
+    __shared__ dfl s_node[3][TIP_N][3], s_pt[3][BOX_S][3];                // parts of the nodes' and the points' positions
+    __shared__ dfl s_wx[XS][TIP_N], s_wy[XS][TIP_N], s_wz[XS][TIP_N];
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nat = prm.ncharged;
+    int b[3], lo[3], hi[3];
+    box_of_cta(prm, B, level, blockIdx.x, b, lo, hi);
+    BoxShare share;
+    bool handed = false;
+    int nlist = -1;
+    if (level < B.levels) {
+        share = box_share<TIP_N, NC>(prm, B, level, b);
+        handed = share_has_sums<TIP_N, NC>(share);
+        if (handed && share.room > 0) nlist = *share_count<TIP_N, NC>(share);
     }
     const int nanc = handed ? B.levels - level : 0;
     const int ncand = nlist >= 0 ? nlist : nat;
     // ---- tables of this box
     if (warp == 1 && lane <= nanc) pk.centre[lane] = box_centre(prm, B, level, b, lane);
-    if (warp == 0 && lane < 24) {
-        const int a = lane >> 3, i = lane & 7;
-        int l, h;
-        box_span(prm, B, level, a, a == 0 ? b[0] : (a == 1 ? b[1] : b[2]), l, h);
-        const dfl g = df_add(df_mul_f(cheb_t(i), box_half(l, h)), {0.5f * (float)(l + h) + (float)prm.i0[a], 0.f});
-#pragma unroll
-        for (int k = 0; k < 3; k++) s_node[a][i][k] = df_mul(B.step[a][k], g);
-    }
-    if (LEAF && tid >= 64 && tid < 64 + 48) {
+    if (warp == 0 && lane < 3 * TIP_N) tip_node_table(prm, B, level, b, lane, s_node);
+    if (tid >= 64 && tid < 64 + 48) {
         const int a = (tid - 64) >> 4, j = (tid - 64) & 15;
         const float g = (float)(prm.i0[a] + (a == 0 ? lo[0] : (a == 1 ? lo[1] : lo[2])) + j);
 #pragma unroll
         for (int k = 0; k < 3; k++) s_pt[a][j][k] = df_mul_f(B.step[a][k], g);
     }
-    for (int i = tid; i < 3 * BOX_S * BOX_N; i += NT) {
-        const int a = i / (BOX_S * BOX_N), pt = (i / BOX_N) % BOX_S, k = i % BOX_N;
-        dfl w;
-        if constexpr (LEAF) {
-            const int m = (a == 0 ? hi[0] - lo[0] : (a == 1 ? hi[1] - lo[1] : hi[2] - lo[2])) + 1;
-            w = {c_cheb_points.w[m][pt][k], c_cheb_points.l[m][pt][k]};
-        } else {
-            w = box_child_weight(prm, B, level, a, a == 0 ? b[0] : (a == 1 ? b[1] : b[2]), pt, k);
-        }
-        (a == 0 ? s_wx : (a == 1 ? s_wy : s_wz))[pt][k] = w;
+    for (int i = tid; i < 3 * XS * TIP_N; i += NT) {
+        const int a = i / (XS * TIP_N), pt = (i / TIP_N) % XS, k = i % TIP_N;
+        const int m = (a == 0 ? hi[0] - lo[0] : (a == 1 ? hi[1] - lo[1] : hi[2] - lo[2])) + 1;
+        (a == 0 ? s_wx : (a == 1 ? s_wy : s_wz))[pt][k] = {cheb_points<TIP_N>().w[m][pt][k], cheb_points<TIP_N>().l[m][pt][k]};
     }
     __syncthreads();
 
-    // ---- far charges on the nodes: thread = half of a node column, one of two parts of the atoms
-    const int sub = tid >> 7, col = (tid & 127) >> 1, half = tid & 1;
+    // ---- far charges on the nodes: a thread has four
+    const bool on_nodes = tid < TIP_N3 / TIP_P;
     dfl p[3][TIP_P];
     TipSums S;
     S.zero();
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const dfl xy = df_add(s_node[0][col >> 3][k], s_node[1][col & 7][k]);
-#pragma unroll
-        for (int i = 0; i < TIP_P; i++)
-            if (k == 2 || i == 0 || !ORTHO) p[k][i] = df_add(xy, s_node[2][4 * half + i][k]);
-    }
+    tip_nodes(s_node, tid, p);
     const bool wide = nat > 65536;
     const int near_cap = wide ? BOX_NEAR / 2 : BOX_NEAR;
     auto near_at = [&](int i) -> int { return wide ? reinterpret_cast<const int *>(s_near)[i] : (int)s_near[i]; };
@@ -265,7 +392,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
         const int i = t * NT + tid;
         int j = -1;
         if (i < (all ? nat : ncand)) {
-            j = all || nlist < 0 ? i : (int)*share_list(share, level, i);
+            j = all || nlist < 0 ? i : (int)*share_list<TIP_N, NC>(share, i);
             box_gather(prm, tiles + ((t & 1) * NT + tid) * FF_REC, j);
         }
         return j;
@@ -273,69 +400,53 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
     for (int t = 0; t < (ncand + NT - 1) / NT; t++) {
         const float4 *T = tiles + (t & 1) * NT * FF_REC;
         const int j0 = gather(t, false);
-        box_pick<M_COUL, NT>(B, pk, level, nanc, T, min(NT, ncand - t * NT), 1, true, nmid, nzero, place);
-        if (place >= 0) {
-            if constexpr (LEAF) {
-                const int i = nnear + place;
-                if (i < near_cap) {
-                    if (wide) reinterpret_cast<int *>(s_near)[i] = j0;
-                    else s_near[i] = (unsigned short)j0;
-                }
-            } else {
-                s_left[place] = (unsigned short)j0;
-            }
+        box_pick<M_COUL, TIP_N, NT>(B, pk, level, nanc, T, min(NT, ncand - t * NT), 1, true, nmid, nzero, place);
+        if (place >= 0 && nnear + place < near_cap) {
+            if (wide) reinterpret_cast<int *>(s_near)[nnear + place] = j0;
+            else s_near[nnear + place] = (unsigned short)j0;
         }
-        __syncthreads();
-        if constexpr (!LEAF) box_leave<NC, NT>(prm, B, level, b, s_left, nzero, nnear);
         nnear += nzero;
-        for (int i = sub; i < nmid; i += 2) {
+        __syncthreads();
+        for (int i = on_nodes ? 0 : nmid; i < nmid; i++) {
             const int j = pk.mid[i];
-            tip_add<KIND, WITH_E, ORTHO>(p, T[3 * j], T[3 * j + 1], T[3 * j + 2].z, S);
+            tip_add<KIND, WITH_E, false>(p, T[3 * j], T[3 * j + 1], T[3 * j + 2].z, S);
         }
         S.fold<WITH_E>();
         __syncthreads();
     }
-    if constexpr (!LEAF) box_leave_count<NC>(prm, B, level, b, nnear);
-    // ---- the nodes' sums: both parts of the atoms and the parent's interpolated sums
-    dfl *nodes = reinterpret_cast<dfl *>(tiles);  // [K][8][8][8]
-    if (sub == 1) {
-#pragma unroll
-        for (int k = 0; k < K; k++)
-#pragma unroll
-            for (int i = 0; i < TIP_P; i++) plane[(k * TIP_P + i) * 128 + (tid & 127)] = S.get(k, i);
-    }
-    __syncthreads();
-    if (sub == 0) {
+    // ---- the nodes' sums and the parent's interpolated sums
+    dfl *nodes = reinterpret_cast<dfl *>(tiles);  // [K][10][10][10]
+    if (on_nodes) {
 #pragma unroll
         for (int k = 0; k < K; k++) {
             dfl v[TIP_P];
 #pragma unroll
-            for (int i = 0; i < TIP_P; i++) v[i] = df_add(S.get(k, i), plane[(k * TIP_P + i) * 128 + tid]);
+            for (int i = 0; i < TIP_P; i++) v[i] = S.get(k, i);
             if (handed) {
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    const float4 o = *share_slot<NC>(share, level, k * 256 + col * 4 + half * 2 + e);
+                    const float4 o = *share_cell(share, k * (TIP_N3 / 2) + 2 * tid + e);
                     v[2 * e] = df_add(v[2 * e], {o.x, o.y});
                     v[2 * e + 1] = df_add(v[2 * e + 1], {o.z, o.w});
                 }
             }
 #pragma unroll
-            for (int i = 0; i < TIP_P; i++) nodes[k * BOX_N3 + col * 8 + half * 4 + i] = v[i];
+            for (int i = 0; i < TIP_P; i++) nodes[k * TIP_N3 + TIP_P * tid + i] = v[i];
         }
     }
     __syncthreads();
-    // ---- along x
-    if (tid < K * 64) {
-        const int k = tid >> 6, r = tid & 63;
-        dfl v[BOX_N];
+    // ---- along x, a thread one node and every other x
+    for (int i = tid; i < 2 * K * TIP_N2; i += NT) {
+        const int x0 = i / (K * TIP_N2), q = i - x0 * (K * TIP_N2), k = q / TIP_N2, r = q - k * TIP_N2;
+        dfl v[TIP_N];
 #pragma unroll
-        for (int a = 0; a < BOX_N; a++) v[a] = nodes[k * BOX_N3 + a * 64 + r];
+        for (int a = 0; a < TIP_N; a++) v[a] = nodes[k * TIP_N3 + a * TIP_N2 + r];
 #pragma unroll 1
-        for (int x = 0; x < BOX_S; x++) {
+        for (int x = x0; x < XS; x += 2) {
             dfl s = {0.f, 0.f};
 #pragma unroll
-            for (int a = 0; a < BOX_N; a++) df_fma(s, s_wx[x][a], v[a]);
-            line[(k * BOX_S + x) * 64 + r] = two_sum(s.h, s.l);
+            for (int a = 0; a < TIP_N; a++) df_fma(s, s_wx[x][a], v[a]);
+            line[(k * XS + x) * TIP_N2 + r] = two_sum(s.h, s.l);
         }
     }
     __syncthreads();
@@ -345,91 +456,76 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
         __syncthreads();
     };
     const bool listed = nnear <= near_cap, staged = nnear <= BOX_STAGE;
-    if (LEAF && listed && staged) stage(0, nnear);
-    const int mx = LEAF ? hi[0] - lo[0] + 1 : BOX_S, my = LEAF ? hi[1] - lo[1] + 1 : BOX_S, mz = hi[2] - lo[2] + 1;
+    if (listed && staged) stage(0, nnear);
+    const int mx = hi[0] - lo[0] + 1, my = hi[1] - lo[1] + 1, mz = hi[2] - lo[2] + 1;
 #pragma unroll 1
-    for (int xh = 0; xh < mx; xh += 8) {
-        // ---- along y, for eight of the box's x
-        __syncthreads();  // the runs of the eight before have read the plane
-        for (int i = tid; i < K * 8 * 16 * 8; i += NT) {
-            const int c = i & 7, y = (i >> 3) & 15, x = (i >> 7) & 7, k = i >> 10;
+    for (int xh = 0; xh < mx; xh += TIP_X) {
+        // ---- along y, for four of the box's x
+        __syncthreads();  // the runs of the four before have read the plane
+        for (int i = tid; i < K * TIP_X * XS * TIP_N; i += NT) {
+            const int c = i % TIP_N, y = i / TIP_N % XS, x = i / (TIP_N * XS) % TIP_X, k = i / (TIP_N * XS * TIP_X);
             dfl s = {0.f, 0.f};
 #pragma unroll
-            for (int a = 0; a < BOX_N; a++) df_fma(s, s_wy[y][a], line[(k * BOX_S + xh + x) * 64 + a * 8 + c]);
+            for (int a = 0; a < TIP_N; a++) df_fma(s, s_wy[y][a], line[(k * XS + xh + x) * TIP_N2 + a * TIP_N + c]);
             plane[i] = two_sum(s.h, s.l);
         }
         __syncthreads();
-        const int nrun = min(8, mx - xh) * my * 4;
+        const int nrun = min(TIP_X, mx - xh) * my * 4;
 #pragma unroll 1
         for (int c0 = 0; c0 < nrun; c0 += NT) {
             const int c = min(c0 + tid, nrun - 1);  // threads past the end repeat the last run and store nothing
             const int h = c & 3, xy = c >> 2, x = xy / my, y = xy - x * my;
-            // ---- along z: leaves every fourth point from h, upper boxes four nodes of a child
+            // ---- along z, every fourth point from h
             S.zero();
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                const dfl *v = plane + ((k * 8 + x) * 16 + y) * 8;
+                const dfl *v = plane + ((k * TIP_X + x) * XS + y) * TIP_N;
 #pragma unroll
                 for (int i = 0; i < TIP_P; i++) {
                     dfl s = {0.f, 0.f};
-                    const dfl *w = s_wz[LEAF ? h + 4 * i : 4 * h + i];
+                    const dfl *w = s_wz[h + 4 * i];
 #pragma unroll
-                    for (int a = 0; a < BOX_N; a++) df_fma(s, w[a], v[a]);
+                    for (int a = 0; a < TIP_N; a++) df_fma(s, w[a], v[a]);
                     s = two_sum(s.h, s.l);
                     if (k == 3) S.E[i] = s;
                     else S.F[k < 3 ? k : 0][i] = s;
                 }
             }
-            if constexpr (!LEAF) {
-                const int ch[3] = {2 * b[0] + ((xh + x) >> 3), 2 * b[1] + (y >> 3), 2 * b[2] + (h >> 1)};
-                if (!box_there(B, level - 1, ch)) continue;
-                const BoxShare cs = box_share<NC>(prm, B, level - 1, ch);
-                if (!share_has_slot<NC>(cs, level - 1)) continue;
 #pragma unroll
-                for (int k = 0; k < K; k++)
+            for (int k = 0; k < 3; k++) {
+                const dfl q = df_add(s_pt[0][xh + x][k], s_pt[1][y][k]);
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const dfl u = S.get(k, 2 * e), w = S.get(k, 2 * e + 1);
-                        *share_slot<NC>(cs, level - 1, k * 256 + (((xh + x) & 7) * 8 + (y & 7)) * 4 + (h & 1) * 2 + e) =
-                            make_float4(u.h, u.l, w.h, w.l);
-                    }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const dfl q = df_add(s_pt[0][xh + x][k], s_pt[1][y][k]);
-#pragma unroll
-                    for (int i = 0; i < TIP_P; i++)
-                        if (k == 2 || i == 0 || !ORTHO) p[k][i] = df_add(q, s_pt[2][h + 4 * i][k]);
+                for (int i = 0; i < TIP_P; i++)
+                    if (k == 2 || i == 0 || !ORTHO) p[k][i] = df_add(q, s_pt[2][h + 4 * i][k]);
+            }
+            if (listed) {
+                for (int n0 = 0; n0 < nnear; n0 += BOX_STAGE) {
+                    const int n1 = min(nnear, n0 + BOX_STAGE);
+                    if (!staged) stage(n0, n1);
+                    for (int j = 0; j < n1 - n0; j++)
+                        tip_add<KIND, WITH_E, ORTHO>(p, tiles[3 * j], tiles[3 * j + 1], tiles[3 * j + 2].z, S);
+                    if (!staged) __syncthreads();
                 }
-                if (listed) {
-                    for (int n0 = 0; n0 < nnear; n0 += BOX_STAGE) {
-                        const int n1 = min(nnear, n0 + BOX_STAGE);
-                        if (!staged) stage(n0, n1);
-                        for (int j = 0; j < n1 - n0; j++)
-                            tip_add<KIND, WITH_E, ORTHO>(p, tiles[3 * j], tiles[3 * j + 1], tiles[3 * j + 2].z, S);
-                        if (!staged) __syncthreads();
+            } else {  // more near atoms than the list holds: through all atoms again
+                for (int t = 0; t < (nat + NT - 1) / NT; t++) {
+                    const float4 *T = tiles + (t & 1) * NT * FF_REC;
+                    gather(t, true);
+                    box_pick<M_COUL, TIP_N, NT>(B, pk, level, nanc, T, min(NT, nat - t * NT), 0, true, nmid, nzero, place);
+                    __syncthreads();
+                    for (int i = 0; i < nmid; i++) {
+                        const int j = pk.mid[i];
+                        tip_add<KIND, WITH_E, ORTHO>(p, T[3 * j], T[3 * j + 1], T[3 * j + 2].z, S);
                     }
-                } else {  // more near atoms than the list holds: through all atoms again
-                    for (int t = 0; t < (nat + NT - 1) / NT; t++) {
-                        const float4 *T = tiles + (t & 1) * NT * FF_REC;
-                        gather(t, true);
-                        box_pick<M_COUL, NT>(B, pk, level, nanc, T, min(NT, nat - t * NT), 0, true, nmid, nzero, place);
-                        __syncthreads();
-                        for (int i = 0; i < nmid; i++) {
-                            const int j = pk.mid[i];
-                            tip_add<KIND, WITH_E, ORTHO>(p, T[3 * j], T[3 * j + 1], T[3 * j + 2].z, S);
-                        }
-                        __syncthreads();
-                    }
+                    __syncthreads();
                 }
-                S.fold<WITH_E>();
-                if (c0 + tid >= nrun) continue;
-                float4 *dst = prm.FE + ((long long)(lo[0] + xh + x) * prm.ns[1] + lo[1] + y) * prm.ns[2] + lo[2] + h;
+            }
+            S.fold<WITH_E>();
+            if (c0 + tid >= nrun) continue;
+            float4 *dst = prm.FE + ((long long)(lo[0] + xh + x) * prm.ns[1] + lo[1] + y) * prm.ns[2] + lo[2] + h;
 #pragma unroll
-                for (int i = 0; i < TIP_P; i++) {
-                    if (h + 4 * i >= mz) break;
-                    tip_store<KIND, WITH_E>(prm, S, i, dst + 4 * i);
-                }
+            for (int i = 0; i < TIP_P; i++) {
+                if (h + 4 * i >= mz) break;
+                tip_store<KIND, WITH_E>(prm, S, i, dst + 4 * i);
             }
         }
     }
@@ -439,41 +535,43 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
 
 template <int KIND, bool WITH_E, bool ORTHO>
 static int launch_tip_boxes(const FFParams &prm, BoxPrm B, cudaStream_t st) {
-    constexpr int smem = (int)tip_box_smem<WITH_E>();
-    PPGPU_CUDA(cudaFuncSetAttribute(tip_box_kernel<KIND, WITH_E, ORTHO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-               "tip boxes' shared memory");
-    PPGPU_CUDA(cudaFuncSetAttribute(tip_box_kernel<KIND, WITH_E, ORTHO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+    constexpr int up = (int)TipUpSmem<WITH_E>::size, leaf = (int)TipSmem<WITH_E>::size;
+    PPGPU_CUDA(cudaFuncSetAttribute(tip_up_kernel<KIND, WITH_E>, cudaFuncAttributeMaxDynamicSharedMemorySize, up), "tip boxes' shared memory");
+    PPGPU_CUDA(cudaFuncSetAttribute(tip_box_kernel<KIND, WITH_E, ORTHO>, cudaFuncAttributeMaxDynamicSharedMemorySize, leaf),
                "tip boxes' shared memory");
     for (B.level = B.levels; B.level >= 0; B.level--) {
         long long n = 1;
         for (int k = 0; k < 3; k++) n *= ((B.nb[k] - 1) >> B.level) + 1;
-        if (n > 0x7fffffffLL) return set_error(PPGPU_ERR_ARG, "ff grid too large (%lld boxes)", n);
-        if (B.level > 0)
-            tip_box_kernel<KIND, WITH_E, ORTHO, false><<<(unsigned)n, TIP_NT, smem, st>>>(prm, B);
-        else
-            tip_box_kernel<KIND, WITH_E, ORTHO, true><<<(unsigned)n, TIP_NT, smem, st>>>(prm, B);
+        if (n > 0x0fffffffLL) return set_error(PPGPU_ERR_ARG, "ff grid too large (%lld boxes)", n);
+        if (B.level > 0) {
+            int rc = launch_box_up(tip_up_kernel<KIND, WITH_E>, up, n, prm, B, st);
+            if (rc) return rc;
+        } else {
+            tip_box_kernel<KIND, WITH_E, ORTHO><<<(unsigned)n, TIP_NT, leaf, st>>>(prm, B);
+            PPGPU_CHECK_LAUNCH("tip_box_kernel launch");
+        }
     }
-    PPGPU_CHECK_LAUNCH("tip_box_kernel launch");
     return set_ok();
 }
 
-// Grids and charges summed by boxes.  dz2, pair by pair against by boxes (0.05 to 0.3 A steps alike
-// where not given): 200^3 points, 342 charges 16.7 against 2.44 ms (3.49 without the level above);
-// 140^3 (729 leaves) 342: 5.84 against 1.95, 90: 1.57 against 0.60, 60: 1.06 against 0.63 (0.05 A) to
-// 1.00 (0.3 A), 30: 0.55 against 0.44 to 0.55; 96^3 (216 leaves) 90: 0.54 against 0.45, 60: 0.37
-// against 0.38 to 0.51; 64^3 (64 leaves) 342: 0.68 against 1.0 to 1.5, the boxes too few for 152 SMs.
-// A level above the leaves: 342 charges gain at 2197 leaves, not at 729 (2.5e5 charge-boxes).
+// Grids and charges summed by boxes.  dz2, pair by pair against by boxes, at 0.1 A steps (in brackets
+// 0.3 A where it differs): 200^3 points (2197 leaves), 342 charges 16.7 against 1.86 ms, 60: 3.02 against
+// 1.33; 140^3 (729) 342: 5.85 against 1.29, 60: 1.07 against 0.67 (0.75), 30: 0.55 against 0.41 (0.45), 6: 0.15
+// against 0.19; 96^3 (216) 342: 1.98 against 1.03, 90: 0.54 against 0.51 (0.71), 60: 0.38 against 0.39 (0.52);
+// 64^3 (64 leaves) 342: 0.69 against 0.83, the boxes too few for 152 SMs.
+//   Levels above the leaves, 0, 1 and 2: 140^3, 90 charges 0.92, 0.94, 0.98 ms (6.6e4 charge-boxes), 96^3, 342 1.22, 1.03,
+// 1.06 (7.4e4), 140^3, 540 3.69, 1.94, 1.99 (3.9e5), 200^3, 342 6.6, 2.15, 1.86 (7.5e5).
 static bool tip_box_rule(const FFParams &prm, double H, BoxPrm *B) {
     const double boxes = (double)B->nb[0] * B->nb[1] * B->nb[2], work = prm.ncharged * boxes;
-    B->levels = prm.accumulate || work < 4e5 ? 0 : (work < 1e8 ? 1 : 2);
-    return boxes >= 200 && H <= 5.0 && prm.ncharged >= 40.0 + 10000.0 / boxes;
+    B->levels = prm.accumulate || work < 7e4 ? 0 : (work < 5e5 ? 1 : (work < 1e8 ? 2 : 3));
+    return boxes >= 200 && H * TIP_KAPPA <= 36.0 && prm.ncharged >= 15.0 + 20000.0 / boxes;
 }
 
 template <int KIND, bool WITH_E, bool ORTHO>
 static int launch_tip(FFParams &prm, cudaStream_t st) {
     BoxPrm B;
     double H;
-    box_plan(prm, TIP_KAPPA, TIP_H, &B, &H);
+    box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, &B, &H);
     if (tip_box_rule(prm, H, &B)) return launch_tip_boxes<KIND, WITH_E, ORTHO>(prm, B, st);
     prm.nzc = (prm.ns[2] + TIP_P - 1) / TIP_P;
     prm.nchunks = (long long)prm.ns[0] * prm.ns[1] * prm.nzc;

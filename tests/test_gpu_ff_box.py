@@ -53,6 +53,14 @@ CASES = [
     ("ljc", (113, 120, 113), 0.1, False, 900, "ball", 0.1, False, False),  # near atoms staged in parts
     ("ljc", (250, 310, 330), 0.1, False, 20000, "slab", 0.97, False, False),  # two levels, parents' lists
     ("lj", (120, 113, 128), 0.1, False, 66000, "slab", 1.0, False, False),  # 32-bit indices, no lists
+    ("ljc", (200, 157, 160), 0.1, True, 400, "plane", 0.3, True, False),  # 8 nodes, one level
+    ("lj", (230, 225, 221), 0.1, False, 1000, "plane", 1.0, False, False),  # 8 nodes, two levels
+    ("ljc", (113, 129, 97), 0.1, True, 300, "plane", 0.5, True, False),  # 10 nodes, one level
+    ("ljc", (200, 200, 170), 0.1, False, 4500, "slab", 0.5, True, False),  # 10 nodes, two levels
+    ("qzs", (130, 120, 110), 0.1, False, 300, "plane", 0.0, False, False),
+    ("lj", (145, 113, 65), 0.1, True, 257, "plane", 1.0, True, False),
+    ("coulomb", (145, 113, 65), 0.3, False, 257, "plane", 0.4, False, False),
+    ("ljc", (113, 129, 97), 0.45, False, 130, "plane", 0.2, False, False),  # 10 nodes for their shorter reach
 ]
 
 
@@ -137,6 +145,30 @@ def test_boxes_atoms_on_grid_points(gpulib):
     for x, y, z in nodes:
         ref = ff.compute_subgrid((x - 1, y - 1, z - 1), (3, 3, 3), rec, na, nch, D.FF_LJC, Q=-0.05, Fmax=10.0).view(3, 3, 3, 4).cpu().numpy()
         assert np.abs(g[x - 1 : x + 2, y - 1 : y + 2, z - 1 : z + 2] - ref).max() <= 1e-5 * 10.0
+
+
+@pytest.mark.parametrize("tilt", [False, True])
+def test_points_near_an_atom(gpulib, tilt):
+    """Grid points 0.03 to 0.06 A from an atom, whose r^-14 shows the rounding of the displacement: its
+    float32 rounding and the reciprocal root's (2^-22.9), 14 times, are 3e-6 of the force and energy."""
+    from ppafm_gb300 import device as D
+
+    n = (113, 129, 97)
+    rng = np.random.default_rng(21)
+    cell = _cell(n, 0.1, tilt)
+    R, c, q = _atoms(rng, 300, cell, "plane")
+    c = np.abs(c)
+    nodes = np.column_stack([rng.integers(2, n[k] - 2, 24) for k in range(3)])
+    d = rng.normal(size=(24, 3))
+    R[:24] = nodes @ (cell / np.array(n)[:, None]) + d / np.linalg.norm(d, axis=1)[:, None] * rng.uniform(0.03, 0.06, (24, 1))
+    rec, na, nch = D.pack_atoms(R, c, None)
+    ff = D.DeviceFF(n, cell)
+    g = ff.compute(rec, na, nch, D.FF_LJ, with_E=True).grid4.cpu().numpy().astype(np.float64)
+    for x, y, z in nodes:
+        ref = ff.compute_subgrid((int(x), int(y), int(z)), (1, 1, 1), rec, na, nch, D.FF_LJ, with_E=True, f64=True).view(4).cpu().numpy().astype(np.float64)
+        got = g[x, y, z]
+        assert np.linalg.norm(got[:3] - ref[:3]) <= 4e-6 * np.linalg.norm(ref[:3])
+        assert abs(got[3] - ref[3]) <= 4e-6 * abs(ref[3])
 
 
 def test_boxes_repeat_bit_for_bit(gpulib):
