@@ -12,8 +12,8 @@ molecule, 800x800x500 grid, 512x512x40 scan (the large single system).
 Printed (rank 0, one JSON line): value = relaxed pixel-heights per second of the whole
 step with the atoms already in device memory; e2e = the same metric through the public
 host API (ppafm_gb300.HighLevel.Pipeline with host atoms in and host fzs/positions/Δf
-out, copies inside the timed region); roofline of the dominant kernel (force field,
-float32-FMA bound) against an FFMA peak measured in the same process; the CPU baseline
+out, copies inside the timed region); roofline of the dominant kernel (force field by
+boxes: the bytes it writes against the measured copy rate); the CPU baseline
 (the reference pipeline on this host's cores, bounded sample, extrapolated).
 
 Multi-GPU (torchrun, N > 1): every rank relaxes its own independent system (weak scaling,
@@ -35,9 +35,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "relaxed pixel-z points/s & FF grid-pt·atoms/s; FIRE iters/pixel at 1e-4 eV/Å"
 UNIT = "pixel-z/s"
-FLOPS_LJ_PAIR = 26  # float32 flops per atom-point pair, FMA = 2 (LJ only)
-FLOPS_LJC_PAIR = 30  # LJ + Coulomb sharing r^2
-FLOPS_TIP_CHARGE_PAIR = 20  # one AFMulator tip charge on one atom (FF.cl evalLJC_QZs_noPos)
+FLOPS_LJC_PAIR = 30  # float32 flops per atom-point pair, FMA = 2 (LJ + Coulomb sharing r^2)
 
 
 def parse():
@@ -141,6 +139,16 @@ def read_measured_peaks():
         return {}
 
 
+def ff_bytes_roofline(name, moved, t_ff):
+    """Roofline of a force field summed by boxes: the bytes it cannot do without (each grid point
+    written, each atom read once) against the measured copy rate.  The pairs it sums are 1/15 (a small
+    molecule) to 1/130 (the slab) of the direct sum's, so the direct sum's flops say nothing here; it
+    is bound by instruction issue."""
+    hbm = read_measured_peaks().get("hbm_gbs")
+    achieved, peak = moved / t_ff / 1e9, hbm or 6800.0
+    return {"bound": "hbm", "kernel": name, "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs" if hbm else "fallback 6800 GB/s", "bytes_per_launch": moved}
+
+
 def ffma_peak_tflops(torch, lib, check, tptr, stream_handle):
     """FP32 FMA peak of this GPU measured now: dependent FFMA chains on every SM."""
     import ctypes
@@ -175,8 +183,8 @@ class PointChargeJob:
         self.npts = int(np.prod(self.pl.gridN))
         self.natoms = self.pl.natoms
         self.nch = self.pl.ncharged
-        self.ff_name = "ff_kernel<LJC> (force field)" if self.pl.Q != 0.0 else "ff_kernel<LJ> (force field)"
-        self.launches_per_step = 2
+        self.ff_name = "ff_box_kernel<LJC> and box_up_kernel (force field by boxes)" if self.pl.Q != 0.0 else "ff_box_kernel<LJ> and box_up_kernel (force field by boxes)"
+        self.launches_per_step = 3 if self.natoms < 5000 else 5  # the leaves, one or three levels of boxes above them, relax
         self.pinned_slots(2)
         self.host_in = {k: np.asarray(w[k]).copy() for k in ("Zs", "Rs", "Qs")}
 
@@ -200,13 +208,8 @@ class PointChargeJob:
         """H2D of the atom records of pinned slot `slot` (on the current stream)."""
         self.pl.atoms.copy_(self.rec_pinned[slot], non_blocking=True)
 
-    def ff_roofline(self, t_ff, peak_fp32):
-        if self.pl.Q != 0.0:
-            flops = self.npts * ((self.natoms - self.nch) * FLOPS_LJ_PAIR + self.nch * FLOPS_LJC_PAIR)
-        else:
-            flops = self.npts * self.natoms * FLOPS_LJ_PAIR
-        achieved = flops / t_ff / 1e12
-        return {"bound": "fp32", "kernel": self.ff_name, "achieved": achieved, "peak": peak_fp32, "unit": "TFLOP/s", "frac": achieved / peak_fp32 if peak_fp32 else None, "peak_source": "FFMA microbenchmark measured in this run (MEASURED_PEAKS.json has no FP32 figure)", "flops_per_launch": flops}
+    def ff_roofline(self, t_ff):
+        return ff_bytes_roofline(self.ff_name, 16.0 * self.npts + 48.0 * self.natoms, t_ff)
 
     def config(self):
         return {"atoms": len(self.w["Zs"]), "atoms_with_images": self.natoms, "charged_atoms_with_images": self.nch}
@@ -224,7 +227,7 @@ class OverlapJob:
         self.torch = torch
         self.pl = HL.DensityOverlapPipeline.from_workload(w, relax=relax, want_iters=False)
         self.npts = int(np.prod(self.pl.gridN))
-        self.launches_per_step = 13  # 2 copies, 2 x (sums + power), 2 x (2 R2C, spectra, C2R x4, pack), R2C + poisson + C2R, relax (cuFFT launches counted as one each)
+        self.launches_per_step = 12  # 2 x (sums + power), 4 R2C, spectra, C2R x4, pack, relax (cuFFT launches counted as one each)
         self.host = [torch.empty(self.pl.gridN, dtype=torch.float32, pin_memory=True) for _ in range(3)]
         for h, d in zip(self.host, (self.pl.rho_s, self.pl.rho_q, self.pl.rho_t)):
             h.copy_(d)
@@ -242,7 +245,7 @@ class OverlapJob:
             d.copy_(h, non_blocking=True)
         return int(sum(h.numel() * h.element_size() for h in self.host))
 
-    def ff_roofline(self, t_ff, peak_fp32):
+    def ff_roofline(self, t_ff):
         return None
 
     def config(self):
@@ -705,10 +708,9 @@ def run_ours(args, rank, world, local):
     # ---------------- roofline of the dominant kernel
     t_ff_avg = float(np.mean(t_ff))
     t_rx_avg = float(np.mean(t_rx))
-    if t_ff_avg >= t_rx_avg and job.ff_roofline(t_ff_avg, 1.0) is not None:
-        peak = ffma_peak_tflops(torch, L, _lib.check, _lib.tptr, _lib.stream_handle)
-        roof = job.ff_roofline(t_ff_avg, peak)
-        roof["traffic"] = read_profile_traffic("ff_kernel", args.workload)
+    if t_ff_avg >= t_rx_avg and job.ff_roofline(t_ff_avg) is not None:
+        roof = job.ff_roofline(t_ff_avg)
+        roof["traffic"] = read_profile_traffic("ff_box_kernel", args.workload)
     else:
         # relaxation: gathers of 8 float4 corners per FIRE iteration + 32 B out per pixel-z
         peaks = read_measured_peaks()
@@ -939,15 +941,9 @@ def run_afmulator(args, rank, world, local):
     iters = int(afm.counter.item())
     _lib.check(L.ppgpu_device_status(_lib.stream_handle()))
     npts = int(np.prod(afm.nDim))
-    # the dominant kernel is the force field (ff_kernel<QZS>, FP32-FMA bound).  Work per
-    # atom-point pair in FF.cl's form (FMA = 2): LJ 26 flops, each nonzero tip charge 20
-    # (offset 1, r^2 5, R2SAFE 1, 1/r^2 1, energy 2, force factor 1, charge weight 3,
-    # accumulation 6): 86 for the three-charge tip
-    nq = int(np.count_nonzero(afm.Qs))
-    flops = float(np.mean([npts * len(z) for _, _, z, _, _ in seen])) * (FLOPS_LJ_PAIR + FLOPS_TIP_CHARGE_PAIR * nq)
-    peak = ffma_peak_tflops(torch, L, _lib.check, _lib.tptr, _lib.stream_handle)
-    achieved = flops / t_ff / 1e12
-    roof = {"bound": "fp32", "kernel": "ff_kernel<QZS> (LJ + point-charge tip force field)", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None, "peak_source": "FFMA microbenchmark measured in this run (MEASURED_PEAKS.json has no FP32 figure)", "flops_per_launch": flops, "flops_per_pair": FLOPS_LJ_PAIR + FLOPS_TIP_CHARGE_PAIR * nq, "traffic": read_profile_traffic("ff_kernel", "afmulator")}
+    natoms = float(np.mean([len(z) for _, _, z, _, _ in seen]))
+    roof = ff_bytes_roofline("ff_box_kernel<QZS> (LJ + point-charge tip force field by boxes)", 16.0 * npts + 48.0 * natoms, t_ff)
+    roof["traffic"] = read_profile_traffic("ff_box_kernel", "afmulator")
     if rank != 0:
         return None
     cpu = None

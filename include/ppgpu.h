@@ -169,7 +169,8 @@ int ppgpu_set_tip_spline(int n, const double *xs, const double *ydys);
  * stroke (same results again).  ppgpu_get_relax_tps returns the value used for nstroke strokes. */
 int ppgpu_set_relax_tps(int tps);
 /* No counterpart in the reference (a launch-shape knob).  Threads per CTA of the single-grid
- * force-field kernel: 128 or 256, 0 = the default (128). */
+ * force-field kernel: 128 or 256, 0 = the default (128). Only for fields
+ * summed pair by pair: larger grids go by boxes, in CTAs of their own size. */
 int ppgpu_set_ff_block(int threads);
 int ppgpu_get_relax_tps(long long nstroke, int *out);
 
