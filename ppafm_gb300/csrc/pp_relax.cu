@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 
+#include "pp_axis_lanes.cuh"
 #include "pp_common.cuh"
 #include "pp_df.cuh"
 #include "pp_relax_dev.cuh"
@@ -278,14 +279,14 @@ __global__ void __launch_bounds__(RELAX_THREADS) relax_kernel(const RelaxPrm P, 
 // now: 32^2 strokes 1.27 -> 0.80 ms, 160^2 1.62 -> 1.37.  The line: one lane with the kept corners
 // against three, 128^2 1.22 against 0.98 ms, 160^2 1.38 against 1.19, 192^2 1.46 against 1.56,
 // 512^2 (40 heights) 6.8 against 8.6.
-constexpr int AXIS_STROKES = 10;  // per warp
 constexpr int AXIS_MAX_STROKES = 30000;  // ~5 warps on each of 608 schedulers
 
 template <bool SCAN>
 __global__ void __launch_bounds__(RELAX_THREADS) relax_axis_kernel(const RelaxPrm P, const StrokeIO S, const ScanIO C) {
     extern __shared__ dfl ztab[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grp = lane / 3, k = lane - 3 * grp, l0 = lane - k;
+    const int warp = threadIdx.x >> 5;
+    const AxisLane al = axis_lane(threadIdx.x & 31);
+    const int k = al.k;
     const int nstroke = SCAN ? C.nx * C.ny : S.nstroke;
     const int nstep = SCAN ? C.nz : S.nstep;
     const dfl dic = k == 0 ? P.dic[0] : (k == 1 ? P.dic[4] : P.dic[8]);
@@ -296,8 +297,8 @@ __global__ void __launch_bounds__(RELAX_THREADS) relax_axis_kernel(const RelaxPr
     const int n = k == 0 ? P.n0 : (k == 1 ? P.n1 : P.n2);
     const int pitch = k == 0 ? P.n1 * P.n2 : (k == 1 ? P.n2 : 1);
     if (SCAN) fill_ztab(ztab, P, C.zs, nstep);
-    const long long s = ((long long)blockIdx.x * (RELAX_THREADS / 32) + warp) * AXIS_STROKES + grp;
-    bool active = grp < AXIS_STROKES && s < nstroke && nstep > 0;
+    const long long s = ((long long)blockIdx.x * (RELAX_THREADS / 32) + warp) * AXIS_STROKES + al.grp;
+    bool active = !al.spare && s < nstroke && nstep > 0;
     const float *fe = reinterpret_cast<const float *>(P.FE) + k;
 
     dfl tip = {0.f, 0.f}, tf = {0.f, 0.f}, d = r0;
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(RELAX_THREADS) relax_axis_kernel(const RelaxPr
     unsigned long long mine = 0;
     float c[8];  // the corner values of the cell that the stroke is in (Corners)
     int cell = -1;
-    auto from = [&](float x, int a) { return __shfl_sync(FULL, x, l0 + a); };
+    auto from = [&](float x, int a) { return __shfl_sync(FULL, x, axis_source(al, a)); };
     auto from_df = [&](dfl x, int a) -> dfl { return {from(x.h, a), from(x.l, a)}; };
 
     while (__any_sync(FULL, active)) {
@@ -347,18 +348,17 @@ __global__ void __launch_bounds__(RELAX_THREADS) relax_axis_kernel(const RelaxPr
             int o[3][2];
 #pragma unroll
             for (int a = 0; a < 3; a++) {
-                o[a][0] = __shfl_sync(FULL, a0, l0 + a);
-                o[a][1] = __shfl_sync(FULL, a1, l0 + a);
+                o[a][0] = __shfl_sync(FULL, a0, axis_source(al, a));
+                o[a][1] = __shfl_sync(FULL, a1, axis_source(al, a));
                 tt[a] = from_df(t, a);
                 const dfl q = fast_two_sum(1.f, -tt[a].h);
                 m[a] = {q.h, __fsub_rn(q.l, tt[a].l)};
             }
-            const int at = o[0][0] + o[1][0] + o[2][0];
+            const int at = axis_corner(o, 0);
             if (at != cell) {
                 cell = at;
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    c[j] = __ldg(fe + 4 * (long long)(o[0][j >> 2] + o[1][(j >> 1) & 1] + o[2][j & 1]));
+                for (int j = 0; j < 8; j++) c[j] = __ldg(fe + 4 * (long long)axis_corner(o, j));
             }
             const dfl wxy[4] = {df_mul(m[0], m[1]), df_mul(m[0], tt[1]), df_mul(tt[0], m[1]), df_mul(tt[0], tt[1])};
             dfl p[8];

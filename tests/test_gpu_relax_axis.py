@@ -62,6 +62,24 @@ def test_axis_scan_matches_one_lane(gpulib, nx, ny, nz, maxIters):
         assert a[k].equal(b[k]), k
 
 
+@pytest.mark.parametrize("r0", [(-0.1, 0.1, 4.0), (0.1, -0.1, 4.0)])
+def test_axis_scan_over_the_whole_cell(gpulib, r0):
+    """A rest position beside the tip, and strokes in every x cell, the last ones too."""
+    from ppafm_gb300 import device as D
+
+    ff = _grid(5)
+    xs, ys = np.arange(N[0]) * 0.2 + 0.05, np.arange(N[1]) * 0.2 + 0.07
+    zs = np.linspace(11.0, 9.0, 12)
+    prm = D.relax_params(maxIters=120, dt=0.5, kRadial=-20.0 / 16.0, kSpring=(-0.0156, -0.0156, 0.0), rPP0=r0)
+
+    def run():
+        return D.relax_scan(ff, prm, xs, ys, zs, want_iters=True)
+
+    a, b = _with_tps(1, run), _with_tps(0, run)
+    for k in a:
+        assert a[k].equal(b[k]), k
+
+
 @pytest.mark.parametrize("probeStart", [-1, 0, 1])
 @pytest.mark.parametrize("relaxAlg", [0, 1])
 @pytest.mark.parametrize("nstroke", [1, 10, 11, 40, 203])
