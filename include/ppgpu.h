@@ -213,6 +213,11 @@ int ppgpu_fft_poisson(void *handle, const float *rho_charge, const double *lvec,
 int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
                              int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
                              void *stream);
+/* The same, and V into a real grid of the plan (NULL: not wanted; untouched without rho_q): what
+ * ppgpu_fft_poisson gives for rho_q, bit for bit. */
+int ppgpu_fft_overlap_forces_v(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
+                               int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
+                               float *V, void *stream);
 
 /* AFMulator Hartree route, cross-correlation (FFTCrossCorrelation.correlate,
  * ppafm/ocl/field.py:800-840): E = IFFT(conj(FFT(rho)) FFT(V)) * scale / N on the plan's grid

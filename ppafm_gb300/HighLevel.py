@@ -581,8 +581,7 @@ class DensityOverlapPipeline:
         self.rho_q = self.fft.empty()
         self.rho_t = self.fft.empty()
         self._ws = self._wt = None  # rho_s^B, rho_t^B of the step-by-step form
-        self._V = self.fft.empty()
-        self._V_done = True
+        self.V = self.fft.empty()
         self.ff = DeviceFF(self.gridN, self.lvec)
         self.prm = tip_vector(parameters, relax)
         xT, yT, zT, self.lvecScan = PPU.prepareScanGrids(_get(parameters, "scanMin"), _get(parameters, "scanMax"), _get(parameters, "scanStep"), _get(parameters, "r0Probe"))
@@ -628,23 +627,12 @@ class DensityOverlapPipeline:
         plain = all(t.dtype == torch.float32 and t.is_cuda and t.is_contiguous() and tuple(t.shape) == self.gridN for t in (self.rho_s, self.rho_q, self.rho_t))
         return plain and not (c - np.diag(np.diag(c))).any()
 
-    @property
-    def V(self):
-        """The Hartree potential of rho_q (V).  The force field of an orthogonal cell does not
-        transform it back, so it is made here on first use after a build_ff."""
-        if not self._V_done:
-            torch.cuda.synchronize()  # the plan's buffers may be in use on another stream
-            self.fft.poisson(self.rho_q, self.lvec, out=self._V)
-            self._V_done = True
-        return self._V
-
     def build_ff(self, stream=None, ff=None):
         """The force field into ``ff`` (default: the pipeline's own grid)."""
         ff = self.ff if ff is None else ff
         g = self.fft
         if self._one_round_trip():
-            self._V_done = self.Q == 0.0  # V stays in the spectrum; the property makes it
-            g.overlap_forces(self.rho_s, self.rho_t, self.rho_q if self.Q != 0.0 else None, self.lvec, ff.FE, B=self.B, fix_negative=self.fix_negative, scale_p=self.A, scale_e=self.Q / self.Ne, stream=stream)
+            g.overlap_forces(self.rho_s, self.rho_t, self.rho_q if self.Q != 0.0 else None, self.lvec, ff.FE, B=self.B, fix_negative=self.fix_negative, scale_p=self.A, scale_e=self.Q / self.Ne, stream=stream, V=self.V)
             return ff
         if self._ws is None:
             self._ws, self._wt = g.empty(), g.empty()
@@ -655,9 +643,8 @@ class DensityOverlapPipeline:
         g.density_power(self._wt, self.B, self.fix_negative, stream=stream)
         g.potential2forces(self._ws, self._wt, self.lvec, FE=ff.FE, scale=self.A, with_E=True, stream=stream)
         if self.Q != 0.0:
-            g.poisson(self.rho_q, self.lvec, out=self._V, stream=stream)
-            self._V_done = True
-            g.potential2forces(self._V, self.rho_t, self.lvec, FE=ff.FE, scale=self.Q / self.Ne, with_E=True, accumulate=True, stream=stream)
+            g.poisson(self.rho_q, self.lvec, out=self.V, stream=stream)
+            g.potential2forces(self.V, self.rho_t, self.lvec, FE=ff.FE, scale=self.Q / self.Ne, with_E=True, accumulate=True, stream=stream)
         return ff
 
     _scan_coords = _scan_coords

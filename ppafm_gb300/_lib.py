@@ -82,6 +82,7 @@ SIGNATURES = {
     "ppgpu_fft_density_power": ([c_void_p, c_void_p, c_double, c_int, c_void_p], c_int),
     "ppgpu_fft_poisson": ([c_void_p, c_void_p, _dp, c_void_p, c_void_p], c_int),
     "ppgpu_fft_overlap_forces": ([c_void_p, c_void_p, c_void_p, c_void_p, c_double, c_int, c_double, c_double, _dp, c_void_p, c_void_p], c_int),
+    "ppgpu_fft_overlap_forces_v": ([c_void_p, c_void_p, c_void_p, c_void_p, c_double, c_int, c_double, c_double, _dp, c_void_p, c_void_p, c_void_p], c_int),
     "ppgpu_fft_correlate": ([c_void_p, c_void_p, c_void_p, c_double, c_void_p, c_void_p], c_int),
     "ppgpu_gaussian_density": ([c_void_p, _ip, _dp, c_int, c_void_p, c_int, c_void_p], c_int),
     "ppgpu_lj_grid_f64_noalloc": ([c_void_p, c_void_p, _ip, _dp, c_int, c_void_p, c_void_p, c_void_p], c_int),

@@ -300,6 +300,16 @@ __device__ __forceinline__ R pois_b(const PoissonPrm &P, int i) {
     else return P.b[i];
 }
 
+// |G|^2 of element (i, j, k) of the half spectrum.
+template <typename R>
+__device__ __forceinline__ R pois_g2(const PoissonPrm &P, int i, int j, int k) {
+    const R m0 = (R)freq(i, P.n0), m1 = (R)freq(j, P.n1), m2 = (R)freq(k, P.n2);
+    const R gx = m0 * pois_b<R>(P, 0) + m1 * pois_b<R>(P, 3) + m2 * pois_b<R>(P, 6);
+    const R gy = m0 * pois_b<R>(P, 1) + m1 * pois_b<R>(P, 4) + m2 * pois_b<R>(P, 7);
+    const R gz = m0 * pois_b<R>(P, 2) + m1 * pois_b<R>(P, 5) + m2 * pois_b<R>(P, 8);
+    return gx * gx + gy * gy + gz * gz;
+}
+
 template <typename C>
 __global__ void poisson_kernel(C *Rk, PoissonPrm P) {
     using R = typename Cx<C>::real;
@@ -308,14 +318,9 @@ __global__ void poisson_kernel(C *Rk, PoissonPrm P) {
     const long long row = q / P.nh2;
     const int k = (int)(q - row * P.nh2);
     const int i = (int)(row / P.n1), j = (int)(row - (long long)i * P.n1);
-    const R m0 = (R)freq(i, P.n0), m1 = (R)freq(j, P.n1), m2 = (R)freq(k, P.n2);
-    const R gx = m0 * pois_b<R>(P, 0) + m1 * pois_b<R>(P, 3) + m2 * pois_b<R>(P, 6);
-    const R gy = m0 * pois_b<R>(P, 1) + m1 * pois_b<R>(P, 4) + m2 * pois_b<R>(P, 7);
-    const R gz = m0 * pois_b<R>(P, 2) + m1 * pois_b<R>(P, 5) + m2 * pois_b<R>(P, 8);
-    const R g2 = gx * gx + gy * gy + gz * gz;
     const C r = Rk[q];
     const R sc = (sizeof(R) == 4) ? (R)P.sf : (R)P.s;
-    const R f = (q == 0) ? (R)0 : sc / g2;
+    const R f = (q == 0) ? (R)0 : sc / pois_g2<R>(P, i, j, k);
     Rk[q] = Cx<C>::make(r.x * f, r.y * f);
 }
 
@@ -323,9 +328,11 @@ __global__ void poisson_kernel(C *Rk, PoissonPrm P) {
 
 struct OverlapPrm {
     SpecPrm sp;
-    PoissonPrm po;       // s, sf: 4 pi k_e, without 1/N (the potential is not transformed back)
+    PoissonPrm po;       // s, sf: 4 pi k_e, without 1/N
+    double vs;           // 4 pi k_e / N, of the potential that is transformed back
+    float vsf;
     double a, q;         // factors of the Pauli and the electrostatic spectra
-    int fix_negative, has_q;
+    int fix_negative, has_q, want_v;
     float B;
     const double *sums;  // [4] sums of rho_s, then of rho_t (fix_negative)
 };
@@ -333,9 +340,10 @@ struct OverlapPrm {
 // The output spectra of the whole density-overlap force field from the four transformed densities:
 // C = a FFT(rho_s^B) conj(FFT(rho_t^B)) + q V conj(FFT(rho_t)), V = 4 pi k_e FFT(rho_q) / G^2, and
 // from C the energy and force spectra as in spectra_kernel.  W, T may be the first two of S4: each
-// thread reads its element of every input before it writes that element.
+// thread reads its element of every input before it writes that element.  want_v: FFT(rho_q) becomes the
+// potential's spectrum, ready for the inverse transform, as in poisson_kernel.
 template <typename C>
-__global__ void overlap_spectra_kernel(const C *W, const C *T, const C *__restrict__ Qk, const C *__restrict__ Rk, C *S4, OverlapPrm P) {
+__global__ void overlap_spectra_kernel(const C *W, const C *T, C *Qk, const C *__restrict__ Rk, C *S4, OverlapPrm P) {
     using R = typename Cx<C>::real;
     __shared__ R s_fac;
     if (threadIdx.x == 0) {
@@ -356,15 +364,16 @@ __global__ void overlap_spectra_kernel(const C *W, const C *T, const C *__restri
     R cr = (w.x * t.x + w.y * t.y) * s_fac;
     R ci = (w.y * t.x - w.x * t.y) * s_fac;
     if (P.has_q) {
-        const R m0 = (R)freq(i, P.po.n0), m1 = (R)freq(j, P.po.n1), m2 = (R)freq(k, P.po.n2);
-        const R gx = m0 * pois_b<R>(P.po, 0) + m1 * pois_b<R>(P.po, 3) + m2 * pois_b<R>(P.po, 6);
-        const R gy = m0 * pois_b<R>(P.po, 1) + m1 * pois_b<R>(P.po, 4) + m2 * pois_b<R>(P.po, 7);
-        const R gz = m0 * pois_b<R>(P.po, 2) + m1 * pois_b<R>(P.po, 5) + m2 * pois_b<R>(P.po, 8);
         const R sc = (sizeof(R) == 4) ? (R)P.po.sf : (R)P.po.s;
-        const R v = (e == 0) ? (R)0 : sc / (gx * gx + gy * gy + gz * gz) * (R)P.q;
+        const R g2 = pois_g2<R>(P.po, i, j, k);
+        const R v = (e == 0) ? (R)0 : sc / g2 * (R)P.q;
         const C q = Qk[e], r = Rk[e];
         cr += v * (q.x * r.x + q.y * r.y);
         ci += v * (q.y * r.x - q.x * r.y);
+        if (P.want_v) {
+            const R f = (e == 0) ? (R)0 : ((sizeof(R) == 4) ? (R)P.vsf : (R)P.vs) / g2;
+            Qk[e] = Cx<C>::make(q.x * f, q.y * f);
+        }
     }
     const R xo = (R)0.5 * (R)rolled_odd2(i, P.sp.n0), yo = (R)0.5 * (R)rolled_odd2(j, P.sp.n1), zo = (R)0.5 * (R)rolled_odd2(k, P.sp.n2);
     const R sE = spec_s<R>(P.sp, false), sF = spec_s<R>(P.sp, true);
@@ -674,12 +683,13 @@ extern "C" int ppgpu_fft_poisson(void *handle, const float *rho_charge, const do
 /* The density-overlap force field in one round trip: FE = scale_p P2F(rho_s^B, rho_t^B) +
  * scale_e P2F(V, rho_t), V the Hartree potential of rho_q (NULL: no electrostatics), energies
  * included, P2F as ppgpu_fft_potential2forces and the densities pre-processed as
- * ppgpu_fft_density_power.  Both parts meet in the spectrum and the potential never leaves it: four
- * transforms forward, four back, where the calls one by one take six and nine (256^3: 1.68 -> 0.93
- * ms, bound by the passes of cuFFT's transforms over memory).  Orthogonal cells. */
-extern "C" int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
-                                        int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
-                                        void *stream) {
+ * ppgpu_fft_density_power.  Both parts meet in the spectrum: four transforms forward, four back, where
+ * the calls one by one take six and nine (256^3: 1.68 -> 0.93 ms, bound by the passes of cuFFT's
+ * transforms over memory); V itself, for a caller who wants it, is a fifth one back (1.02 ms).
+ * Orthogonal cells. */
+extern "C" int ppgpu_fft_overlap_forces_v(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
+                                          int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
+                                          float *V, void *stream) {
     FFTPlan *P = (FFTPlan *)handle;
     if (!P || !rho_s || !rho_t || !lvec || !FE) return set_error(PPGPU_ERR_ARG, "overlap_forces: null argument");
     if (lvec[4] != 0.0 || lvec[5] != 0.0 || lvec[6] != 0.0 || lvec[8] != 0.0 || lvec[9] != 0.0 || lvec[10] != 0.0)
@@ -692,6 +702,9 @@ extern "C" int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const 
     op.q = scale_e;
     op.fix_negative = fix_negative ? 1 : 0;
     op.has_q = rho_q ? 1 : 0;
+    op.want_v = rho_q && V ? 1 : 0;
+    op.vs = op.po.s * (1.0 / (double)P->N);
+    op.vsf = (float)op.vs;
     op.B = (float)B;
     op.sums = P->sums;
     PPGPU_CUFFT(cufftSetStream(P->r2c, st), "cufftSetStream");
@@ -720,21 +733,36 @@ extern "C" int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const 
     }
     if (P->f64) {
         overlap_spectra_kernel<cufftDoubleComplex><<<spec_blocks(P), FFT_THREADS, 0, st>>>(
-            (const cufftDoubleComplex *)Wk, (const cufftDoubleComplex *)Tk, (const cufftDoubleComplex *)P->Vk,
+            (const cufftDoubleComplex *)Wk, (const cufftDoubleComplex *)Tk, (cufftDoubleComplex *)P->Vk,
             (const cufftDoubleComplex *)P->Rk, (cufftDoubleComplex *)P->S4, op);
         PPGPU_CHECK_LAUNCH("overlap_spectra_kernel");
         PPGPU_CUFFT(cufftExecZ2D(P->c2r4, (cufftDoubleComplex *)P->S4, (double *)P->planar), "inverse x4");
         pack_fe_kernel<double><<<blocks_for(P->N), FFT_THREADS, 0, st>>>((float4 *)FE, (const double *)P->planar, P->N, 1.0, 1, 0);
     } else {
         overlap_spectra_kernel<cufftComplex><<<spec_blocks(P), FFT_THREADS, 0, st>>>(
-            (const cufftComplex *)Wk, (const cufftComplex *)Tk, (const cufftComplex *)P->Vk, (const cufftComplex *)P->Rk,
+            (const cufftComplex *)Wk, (const cufftComplex *)Tk, (cufftComplex *)P->Vk, (const cufftComplex *)P->Rk,
             (cufftComplex *)P->S4, op);
         PPGPU_CHECK_LAUNCH("overlap_spectra_kernel");
         PPGPU_CUFFT(cufftExecC2R(P->c2r4, (cufftComplex *)P->S4, (cufftReal *)P->planar), "inverse x4");
         pack_fe_kernel<float><<<blocks_for(P->N), FFT_THREADS, 0, st>>>((float4 *)FE, (const float *)P->planar, P->N, 1.0, 1, 0);
     }
     PPGPU_CHECK_LAUNCH("pack_fe_kernel");
+    if (!op.want_v) return set_ok();
+    PPGPU_CUFFT(cufftSetStream(P->c2r1, st), "cufftSetStream");
+    if (P->f64) {  // the planes are packed: free again
+        PPGPU_CUFFT(cufftExecZ2D(P->c2r1, (cufftDoubleComplex *)P->Vk, stage), "inverse V");
+        f64_to_f32_kernel<<<blocks_for(P->N), FFT_THREADS, 0, st>>>(V, stage, P->N);
+        PPGPU_CHECK_LAUNCH("f64_to_f32_kernel");
+    } else {
+        PPGPU_CUFFT(cufftExecC2R(P->c2r1, (cufftComplex *)P->Vk, (cufftReal *)V), "inverse V");
+    }
     return set_ok();
+}
+
+extern "C" int ppgpu_fft_overlap_forces(void *handle, const float *rho_s, const float *rho_t, const float *rho_q, double B,
+                                        int fix_negative, double scale_p, double scale_e, const double *lvec, float *FE,
+                                        void *stream) {
+    return ppgpu_fft_overlap_forces_v(handle, rho_s, rho_t, rho_q, B, fix_negative, scale_p, scale_e, lvec, FE, nullptr, stream);
 }
 
 extern "C" int ppgpu_gaussian_density(float *rho, const int *n, const double *lvec, int natoms, const double *atoms,

@@ -90,12 +90,12 @@ class FFTGrid:
         check(lib().ppgpu_fft_poisson(self.handle, tptr(rho_charge.contiguous()), dptr(_lvec4(lvec)), tptr(out), stream_handle(stream)))
         return out
 
-    def overlap_forces(self, rho_s, rho_t, rho_q, lvec, FE, B=1.0, fix_negative=True, scale_p=1.0, scale_e=1.0, stream=None):
+    def overlap_forces(self, rho_s, rho_t, rho_q, lvec, FE, B=1.0, fix_negative=True, scale_p=1.0, scale_e=1.0, stream=None, V=None):
         """FE = scale_p * potential2forces(rho_s^B, rho_t^B) + scale_e * potential2forces(V, rho_t), V
         the Hartree potential of rho_q (None: the first part alone), in one round trip; orthogonal
-        cells."""
-        check(lib().ppgpu_fft_overlap_forces(self.handle, tptr(rho_s.contiguous()), tptr(rho_t.contiguous()), None if rho_q is None else tptr(rho_q.contiguous()), float(B), 1 if fix_negative else 0,
-                                             float(scale_p), float(scale_e), dptr(_lvec4(lvec)), tptr(FE), stream_handle(stream)))
+        cells.  V: a grid that the potential is written to as well."""
+        check(lib().ppgpu_fft_overlap_forces_v(self.handle, tptr(rho_s.contiguous()), tptr(rho_t.contiguous()), None if rho_q is None else tptr(rho_q.contiguous()), float(B), 1 if fix_negative else 0,
+                                               float(scale_p), float(scale_e), dptr(_lvec4(lvec)), tptr(FE), tptr(V), stream_handle(stream)))
         return FE
 
     def correlate(self, V, rho, scale=1.0, out=None, stream=None):

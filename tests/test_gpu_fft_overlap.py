@@ -88,3 +88,41 @@ def test_overlap_forces_rejects_skewed_cells(gpulib):
     FE = torch.empty(g.N * 4, device="cuda")
     with pytest.raises(PPGPUError, match="orthogonal"):
         g.overlap_forces(r, r, None, np.array([[4.0, 0, 0], [0.5, 4, 0], [0, 0, 4]]), FE)
+
+
+@pytest.mark.parametrize("f64", [False, True])
+def test_potential_is_that_of_the_last_build(gpulib, f64):
+    """V, one buffer for the pipeline's life, holds the potential that the last build_ff used: bit for
+    bit poisson's, whatever happened to the densities since, on any stream, captured or not."""
+    import torch
+
+    from ppafm_gb300 import HighLevel, workloads
+
+    pl = HighLevel.DensityOverlapPipeline.from_workload(workloads.density_overlap(seed=2, scale=0.15), f64=f64)
+    assert pl._one_round_trip() and pl.Q != 0.0
+    V = pl.V
+    pl.build_ff()
+    first = V.clone()
+    assert first.equal(pl.fft.poisson(pl.rho_q, pl.lvec))
+    keep = [t.clone() for t in (pl.rho_s, pl.rho_q, pl.rho_t)]
+    pl.set_densities(keep[0], 2.0 * keep[1].roll(3, 0), keep[2])
+    assert pl.V is V and V.equal(first)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    pl.build_ff(stream=s)
+    torch.cuda.current_stream().wait_stream(s)
+    second = V.clone()
+    assert second.equal(pl.fft.poisson(pl.rho_q, pl.lvec)) and not second.equal(first)
+    pl.set_densities(*keep)
+    torch.cuda.synchronize()
+    out = torch.zeros_like(V)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        pl.build_ff()
+        out.copy_(pl.V)
+    g.replay()
+    torch.cuda.synchronize()
+    assert out.equal(first) and V.equal(first)
+    pl.V = torch.zeros_like(V)  # another buffer of the caller's
+    pl.build_ff()
+    assert pl.V.equal(first)
