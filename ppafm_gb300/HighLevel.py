@@ -580,7 +580,8 @@ class DensityOverlapPipeline:
         self.rho_s = self.fft.empty()
         self.rho_q = self.fft.empty()
         self.rho_t = self.fft.empty()
-        self._ws = self._wt = None  # rho_s^B, rho_t^B of the step-by-step form
+        self._ws = self.fft.empty()  # rho_s^B of the step-by-step form
+        self._wt = self.fft.empty()  # rho_t^B
         self.V = self.fft.empty()
         self.ff = DeviceFF(self.gridN, self.lvec)
         self.prm = tip_vector(parameters, relax)
@@ -634,8 +635,6 @@ class DensityOverlapPipeline:
         if self._one_round_trip():
             g.overlap_forces(self.rho_s, self.rho_t, self.rho_q if self.Q != 0.0 else None, self.lvec, ff.FE, B=self.B, fix_negative=self.fix_negative, scale_p=self.A, scale_e=self.Q / self.Ne, stream=stream, V=self.V)
             return ff
-        if self._ws is None:
-            self._ws, self._wt = g.empty(), g.empty()
         with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
             self._ws.copy_(self.rho_s)
             self._wt.copy_(self.rho_t)

@@ -126,3 +126,24 @@ def test_potential_is_that_of_the_last_build(gpulib, f64):
     pl.V = torch.zeros_like(V)  # another buffer of the caller's
     pl.build_ff()
     assert pl.V.equal(first)
+
+
+def test_step_by_step_form_allocates_nothing(gpulib):
+    """A skewed cell's build_ff, the first one too and on a stream of its own, works in the pipeline's
+    buffers: memory taken from the current stream's pool there could still be in use."""
+    import torch
+
+    from ppafm_gb300 import HighLevel, workloads
+
+    w = workloads.density_overlap(seed=3, scale=0.12)
+    lvec = np.array(w["lvec"], dtype=np.float64)
+    lvec[2, 0] += 0.2 * lvec[1, 0]
+    pl = HighLevel.DensityOverlapPipeline.from_workload(dict(w, lvec=lvec))
+    assert not pl._one_round_trip()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    before = torch.cuda.memory_allocated()
+    pl.build_ff(stream=s)
+    assert torch.cuda.memory_allocated() == before
+    s.synchronize()
+    assert bool(torch.isfinite(pl.ff.FE).all())
