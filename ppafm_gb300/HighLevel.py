@@ -443,12 +443,19 @@ class StepPipeline:
                 ev[1].record(sf)
         with torch.cuda.stream(sr):
             sr.wait_event(ff_done)
-            if self._out_free[j] is not None:
-                sr.wait_event(self._out_free[j])
+            self._rx_start = torch.cuda.Event()
+            # The reader of an output set may be slow: it holds back the relaxation that writes there,
+            # not the next force field.
+            free = self._out_free[j]
+            early = free is not None and (before_relax is None or not free.query())
+            if early:
+                self._rx_start.record(sr)
+            if free is not None:
+                sr.wait_event(free)
             if before_relax is not None:
                 before_relax()
-            self._rx_start = torch.cuda.Event()
-            self._rx_start.record(sr)
+            if not early:
+                self._rx_start.record(sr)
             if ev:
                 ev[2].record(sr)
             out = self.pl.relax(stream=sr, ff=self.ffs[j], out=self.outs[j])

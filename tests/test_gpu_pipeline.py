@@ -212,3 +212,35 @@ def test_step_pipeline_matches_run(gpulib):
     for k, got in enumerate(steps):
         for key, v in ref[k % 2].items():
             assert torch.equal(got[key], v), (k, key)
+
+
+@pytest.mark.parametrize("hook", [False, True])
+def test_step_pipeline_slow_reader(gpulib, hook):
+    """A reader that has not released its output set holds back the relaxation that writes there, not
+    the force field of the step after it."""
+    import torch
+
+    from ppafm_gb300 import HighLevel as HL
+    from ppafm_gb300 import workloads
+
+    w = workloads.small_molecule(seed=2, scale=0.2)
+    relax = dict(maxIters=w["maxIters"], convF2=w["convF2"], dt=w["dt"], damping=w["damping"])
+    pl = HL.Pipeline(w["Zs"], w["Rs"], w["Qs"], w["lvec"], w["gridN"], w, relax=relax)
+    sp = HL.StepPipeline(pl)
+    before_relax = (lambda: None) if hook else None
+    for _ in range(3):
+        sp.step(before_relax=before_relax)
+    sp.wait_idle()
+    torch.cuda.synchronize()
+    reader = torch.cuda.Stream()
+    end = torch.cuda.Event(enable_timing=True)
+    with torch.cuda.stream(reader):
+        torch.cuda._sleep(400_000_000)  # ~0.2 s
+        end.record(reader)
+    sp.release(sp.k % sp.nbuf, end)
+    held, free = [], []
+    sp.step(timing=held, before_relax=before_relax)
+    sp.step(timing=free, before_relax=before_relax)
+    torch.cuda.synchronize()
+    assert end.elapsed_time(held[0][2]) >= 0  # its relaxation waited
+    assert free[0][1].elapsed_time(end) > 0  # the next step's force field did not
