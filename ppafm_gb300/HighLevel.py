@@ -414,7 +414,8 @@ class StepPipeline:
         self._grid_free = [None] * nbuf  # relaxation that last read grid j
         self._out_free = [None] * nbuf  # consumer of output set j (released)
         self._rx_start = None  # the last step's relaxation is about to start
-        self._tick = torch.zeros(1, device=pl.ff.FE.device)
+        with torch.cuda.stream(self.s_ff):  # of that stream's memory, which has it back in order
+            self._tick = torch.zeros(1, device=pl.ff.FE.device)
         self.k = 0
 
     def step(self, after=None, timing=None, before_relax=None):

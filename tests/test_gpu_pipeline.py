@@ -244,3 +244,29 @@ def test_step_pipeline_slow_reader(gpulib, hook):
     torch.cuda.synchronize()
     assert end.elapsed_time(held[0][2]) >= 0  # its relaxation waited
     assert free[0][1].elapsed_time(end) > 0  # the next step's force field did not
+
+
+def test_step_pipeline_may_go_before_its_steps(gpulib):
+    """Steps that are still queued when their StepPipeline is gone write to no memory that others have
+    by then: what it works in besides its grids and outputs is its own stream's."""
+    import torch
+
+    from ppafm_gb300 import HighLevel as HL
+    from ppafm_gb300 import workloads
+
+    w = workloads.small_molecule(seed=2, scale=0.2)
+    relax = dict(maxIters=w["maxIters"], convF2=w["convF2"], dt=w["dt"], damping=w["damping"])
+    pl = HL.Pipeline(w["Zs"], w["Rs"], w["Qs"], w["lvec"], w["gridN"], w, relax=relax)
+    sp = HL.StepPipeline(pl)
+    kept = [sp.ffs, sp.outs, sp.s_ff, sp.s_rx]  # the caller's results
+    for _ in range(2):
+        sp.step()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(sp.s_ff):
+        torch.cuda._sleep(100_000_000)  # ~50 ms: the steps below are queued behind it
+    for _ in range(2):
+        sp.step()
+    del sp
+    mine = [torch.full((1,), 5.0, device="cuda") for _ in range(64)]
+    torch.cuda.synchronize()
+    assert all(float(t) == 5.0 for t in mine) and len(kept) == 4
