@@ -551,7 +551,9 @@ extern "C" int ppgpu_lj_grid_f64_noalloc(double *gridF, double *gridE, const int
             prm.ns[1] = nbk;
             prm.ns[2] = n[2];
             prm.accumulate = 0;
-            if ((st = ff_dispatch(prm, PPGPU_FF_LJ, 0, with_e, ortho, cs))) return st;
+            // Pair by pair whatever the sizes: the kernels that a first small call loads are all that
+            // any later one needs.
+            if ((st = launch_ff_e<M_LJ, 4>(prm, with_e, ortho, cs))) return st;
             const long long off = ((long long)ia * n[1] + ib) * n[2];
             const long long m = (long long)na_ * nbk * n[2];
             if ((st = ppgpu_grid_to_f64(gridF ? gridF + 3 * off : nullptr, gridE ? gridE + off : nullptr, chunk, m, 1,

@@ -102,3 +102,56 @@ def test_noalloc_rejects_oversized_requests(gpulib):
     big = np.array([1, 1, 300000], np.int32)
     st = L.ppgpu_lj_grid_f64_noalloc(_lib.tptr(F), None, _lib.iptr(big), _lib.dptr(cell), 1, _lib.tptr(R), _lib.tptr(c), _lib.stream_handle())
     assert st == _lib.PPGPU_ERR_ARG
+
+
+MANY = np.array([60, 200, 200], np.int32)  # 6-plane chunks of 169 boxes of 16^3
+
+
+def _many():
+    """Atoms and a grid that the allocating entry points would sum by boxes."""
+    rng = np.random.default_rng(5)
+    lvec = np.array([[0.0, 0, 0], [6.0, 0, 0], [0, 20.0, 0], [0, 0, 20.0]])
+    R = np.column_stack([rng.uniform(-4, 10, 900), rng.uniform(0, 20, 900), rng.uniform(-6, 0.0, 900)])
+    return lvec, R, np.column_stack([rng.uniform(10, 60, 900), rng.uniform(1e4, 8e4, 900)])
+
+
+def test_noalloc_many_atoms_is_the_direct_sum(gpulib):
+    """Pair by pair at every size: bit for bit the columns that the device API sums pair by pair
+    (too few points for boxes)."""
+    from ppafm_gb300 import device as D
+
+    lvec, R, c = _many()
+    F, E, _, _ = _noalloc(gpulib, MANY, lvec, [(R, c)], True)
+    rec, na, nch = D.pack_atoms(R, c, None)
+    ff = D.DeviceFF((2, 2, 2), lvec)
+    ff.n = MANY  # the grid that the sub-boxes are taken from; no whole grid is needed
+    for i0 in [(0, 0, 0), (5, 31, 0), (6, 100, 0), (57, 193, 0)]:
+        g = ff.compute_subgrid(i0, (3, 7, 200), rec, na, nch, D.FF_LJ, with_E=True).view(3, 7, 200, 4).cpu().numpy().astype(np.float64)
+        at = np.s_[i0[0] : i0[0] + 3, i0[1] : i0[1] + 7]
+        assert (F[at] == g[..., :3]).all() and (E[at] == g[..., 3]).all()
+
+
+def test_noalloc_after_one_small_call(gpulib):
+    """In a process of its own, where nothing else has loaded device code: one small call, and a large
+    one with many atoms takes no device memory."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import numpy as np, torch
+from ppafm_gb300 import _lib
+from tests.test_zz_no_alloc import MANY, _many, _noalloc
+L = _lib.load()
+lvec, R, c = _many()
+small = np.array([4, 4, 4], np.int32)
+cell = lvec * 0.1
+_noalloc(L, small, cell, [(R[:3], c[:3])], True)
+torch.zeros(int(MANY.prod()) * 4, dtype=torch.float64, device="cuda")  # the pool that the call's buffers come from
+F, E, free0, free1 = _noalloc(L, MANY, lvec, [(R, c)], True)
+assert free0 == free1, (free0, free1)
+assert np.isfinite(F).all()
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
