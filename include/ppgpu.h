@@ -125,6 +125,12 @@ int ppgpu_ff_subgrid(float *FE, const int *n, const double *cell, const int *i0,
                      const float *atoms, int natoms, int ncharged, int mode, int coul_kind, double Q,
                      double Fmax, const double *Qs, const double *QZs, int flags, void *stream);
 
+/* How a call with these arguments sums its field (host only, no GPU needed): out[0] nodes per axis of
+ * its boxes, 0 for pair by pair; out[1] levels of boxes above the leaves.  It depends on the sizes, so a
+ * sub-box of a grid may be summed another way than the grid, and agree to the rounding only. */
+int ppgpu_ff_route(const int *n, const double *cell, const int *ns, int natoms, int ncharged, int mode, int coul_kind,
+                   const double *Qs, const double *QZs, int flags, int *out);
+
 /* ------------------------------------------------------------------- relaxation
  * Tip/relaxation parameters shared by the relax entry points (float64, host):
  *   prm[0]  maxIters        prm[1] convF2    prm[2] dt (= dtmax)  prm[3] damping (= acoef0)

@@ -310,14 +310,10 @@ extern "C" int ppgpu_pack_atoms(int natoms, const double *R, const double *cLJ, 
     return set_ok();
 }
 
-extern "C" int ppgpu_ff_subgrid(float *FE, const int *n, const double *cell, const int *i0, const int *ns,
-                                const float *atoms, int natoms, int ncharged, int mode, int coul_kind, double Q,
-                                double Fmax, const double *Qs, const double *QZs, int flags, void *stream) {
-    if (!FE || !n || !cell || !i0 || !ns) return set_error(PPGPU_ERR_ARG, "ff_grid: null argument");
+// The checks and parameters of a force-field call, without its buffers.
+static int ff_params(FFParams &prm, const int *n, const double *cell, const int *i0, const int *ns, int natoms, int ncharged,
+                     int mode, int coul_kind, double Q, double Fmax, const double *Qs, const double *QZs, int flags) {
     if (natoms < 0 || ncharged < 0 || ncharged > natoms) return set_error(PPGPU_ERR_ARG, "ff_grid: bad atom counts");
-    if (natoms > 0 && !atoms) return set_error(PPGPU_ERR_ARG, "ff_grid: null atoms");
-    if (((uintptr_t)atoms & 15u) != 0 || ((uintptr_t)FE & 15u) != 0)
-        return set_error(PPGPU_ERR_ARG, "ff_grid: atoms and FE must be 16-byte aligned");
     for (int k = 0; k < 3; k++) {
         if (n[k] <= 0 || ns[k] < 0 || i0[k] < 0 || i0[k] + ns[k] > n[k])
             return set_error(PPGPU_ERR_ARG, "ff_grid: bad grid/sub-box on axis %d", k);
@@ -329,10 +325,7 @@ extern "C" int ppgpu_ff_subgrid(float *FE, const int *n, const double *cell, con
     GridGeom g;
     int st = make_geom(n, cell, &g);
     if (st) return st;
-    FFParams prm;
     memset(&prm, 0, sizeof(prm));
-    prm.FE = reinterpret_cast<float4 *>(FE);
-    prm.atoms = reinterpret_cast<const float4 *>(atoms);
     prm.natoms = natoms;
     prm.ncharged = ncharged;
     for (int k = 0; k < 3; k++) {
@@ -373,9 +366,24 @@ extern "C" int ppgpu_ff_subgrid(float *FE, const int *n, const double *cell, con
         }
     }
     prm.accumulate = (flags & PPGPU_FF_ACCUMULATE) ? 1 : 0;
+    return PPGPU_OK;
+}
+
+extern "C" int ppgpu_ff_subgrid(float *FE, const int *n, const double *cell, const int *i0, const int *ns,
+                                const float *atoms, int natoms, int ncharged, int mode, int coul_kind, double Q,
+                                double Fmax, const double *Qs, const double *QZs, int flags, void *stream) {
+    if (!FE || !n || !cell || !i0 || !ns) return set_error(PPGPU_ERR_ARG, "ff_grid: null argument");
+    if (natoms > 0 && !atoms) return set_error(PPGPU_ERR_ARG, "ff_grid: null atoms");
+    if (((uintptr_t)atoms & 15u) != 0 || ((uintptr_t)FE & 15u) != 0)
+        return set_error(PPGPU_ERR_ARG, "ff_grid: atoms and FE must be 16-byte aligned");
+    FFParams prm;
+    int st = ff_params(prm, n, cell, i0, ns, natoms, ncharged, mode, coul_kind, Q, Fmax, Qs, QZs, flags);
+    if (st) return st;
+    prm.FE = reinterpret_cast<float4 *>(FE);
+    prm.atoms = reinterpret_cast<const float4 *>(atoms);
     prm.err = device_error_word();
     const bool with_e = (flags & PPGPU_FF_WITH_E) != 0;
-    const bool ortho = (g.dcell[6] == 0.0 && g.dcell[7] == 0.0);
+    const bool ortho = (prm.dC[0] == 0.0 && prm.dC[1] == 0.0);
     if ((long long)ns[0] * ns[1] * ns[2] == 0) return set_ok();
     if (mode == PPGPU_FF_COULOMB && ncharged == 0 && !prm.accumulate) {
         // Nothing charged: the grid is exactly zero (plus nothing to add when accumulating).
@@ -384,6 +392,21 @@ extern "C" int ppgpu_ff_subgrid(float *FE, const int *n, const double *cell, con
     }
     if (flags & PPGPU_FF_F64) return ff64_dispatch(prm, mode, coul_kind, (cudaStream_t)stream);
     return ff_dispatch(prm, mode, coul_kind, with_e, ortho, (cudaStream_t)stream);
+}
+
+extern "C" int ppgpu_ff_route(const int *n, const double *cell, const int *ns, int natoms, int ncharged, int mode,
+                              int coul_kind, const double *Qs, const double *QZs, int flags, int *out) {
+    if (!n || !cell || !ns || !out) return set_error(PPGPU_ERR_ARG, "ff_route: null argument");
+    const int zero[3] = {0, 0, 0};
+    FFParams prm;
+    int st = ff_params(prm, n, cell, zero, ns, natoms, ncharged, mode, coul_kind, 0.0, 0.0, Qs, QZs, flags);
+    if (st) return st;
+    const bool tip = mode == PPGPU_FF_COULOMB && coul_kind != 0;
+    FFRoute r = {0, 0};
+    if (!(flags & PPGPU_FF_F64)) r = tip ? ff_tip_route(prm) : ff_box_route(prm, mode, (flags & PPGPU_FF_WITH_E) != 0);
+    out[0] = r.nodes;
+    out[1] = r.levels;
+    return set_ok();
 }
 
 extern "C" int ppgpu_set_ff_block(int threads) {

@@ -67,6 +67,12 @@ bool ff_box_rule(const FFParams &prm, int mode, bool with_e) {
     return box_choice(prm, mode, with_e, &B).boxes;
 }
 
+FFRoute ff_box_route(const FFParams &prm, int mode, bool with_e) {
+    BoxPrm B;
+    const BoxChoice c = box_choice(prm, mode, with_e, &B);
+    return c.boxes ? FFRoute{c.N, B.levels} : FFRoute{0, 0};
+}
+
 int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st) {
     BoxPrm B;
     return box_choice(prm, mode, with_e, &B).N == 8 ? launch_box_nodes<8>(prm, B, mode, with_e, ortho, st) : launch_ff_box10(prm, B, mode, with_e, ortho, st);

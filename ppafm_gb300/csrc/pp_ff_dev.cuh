@@ -52,6 +52,12 @@ inline void ff_set_offsets(FFParams &prm) {
 // Force fields by boxes (pp_ff_box.cu): whether a grid and its atoms are summed that way.
 bool ff_box_rule(const FFParams &prm, int mode, bool with_e);
 int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st);
+// Nodes per axis of its boxes (0: pair by pair) and levels of boxes above the leaves.
+struct FFRoute {
+    int nodes, levels;
+};
+FFRoute ff_box_route(const FFParams &prm, int mode, bool with_e);
+FFRoute ff_tip_route(const FFParams &prm);
 // The pz (1) and dz2 (2) Coulomb tips in double-float (pp_ff_tip.cu).
 int launch_ff_tip(FFParams &prm, int kind, bool with_e, bool ortho, cudaStream_t st);
 

@@ -567,6 +567,13 @@ static bool tip_box_rule(const FFParams &prm, double H, BoxPrm *B) {
     return boxes >= 200 && H * TIP_KAPPA <= 36.0 && prm.ncharged >= 15.0 + 20000.0 / boxes;
 }
 
+FFRoute ff_tip_route(const FFParams &prm) {
+    BoxPrm B;
+    double H;
+    box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, &B, &H);
+    return tip_box_rule(prm, H, &B) ? FFRoute{TIP_N, B.levels} : FFRoute{0, 0};
+}
+
 template <int KIND, bool WITH_E, bool ORTHO>
 static int launch_tip(FFParams &prm, cudaStream_t st) {
     BoxPrm B;

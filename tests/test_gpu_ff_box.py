@@ -115,6 +115,16 @@ def test_boxes_match_float64(gpulib, case):
             assert (g[..., 3] == 0).all()
 
 
+MORE = [
+    ("ljc", (113, 129, 97), 0.1, True, 1300, "plane", 0.5, True, False),  # 10 nodes with the energy, a tilted cell
+]
+
+
+@pytest.mark.parametrize("case", MORE, ids=lambda c: "-".join(map(str, (c[0], *c[1], c[4], c[5]))))
+def test_more_boxes_match_float64(gpulib, case):
+    test_boxes_match_float64(gpulib, case)
+
+
 def _subgrid_f64(ff, i0, ns, rec, na, nch, mode, Q, Fmax, flags, tip):
     """A sub-box of the grid in float64 (compute_subgrid has no tip charges)."""
     import torch
