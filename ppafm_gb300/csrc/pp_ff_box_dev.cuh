@@ -21,6 +21,18 @@ constexpr int BOX_STAGE = BOX_NT;       // near atoms staged at a time
 constexpr int BOX_LEFT = 4096;          // atoms that a CTA of an upper box leaves to the children
 constexpr int BOX_NEAR = 1024;          // near atoms listed, as 16-bit indices (half of it as 32-bit ones)
 
+// Indices of a leaf's near atoms, in either width (wide: more than 65536 atoms).
+union BoxNear {
+    unsigned short h[BOX_NEAR];
+    int w[BOX_NEAR / 2];
+    __device__ __forceinline__ int at(bool wide, int i) const { return wide ? w[i] : (int)h[i]; }
+    __device__ __forceinline__ void set(bool wide, int i, int j) {
+        if (wide) w[i] = j;
+        else h[i] = (unsigned short)j;
+    }
+};
+static_assert(alignof(BoxNear) == alignof(int), "32-bit access");
+
 struct BoxPrm {
     int s[3];    // points of a leaf along an axis, one more for the first rem[axis] leaves; the last may have fewer
     int rem[3];

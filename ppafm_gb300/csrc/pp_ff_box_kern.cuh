@@ -106,10 +106,10 @@ __device__ __forceinline__ void box_add(const FFParams &prm, const BoxPrm &B, co
 // Rare: a point whose float32 sums overflow, within ~5e-3 A of an atom: the far sums t (and u) and
 // the listed near atoms (charged ones first) with r^2 floored like ff_block's slow path.
 template <int MODE, bool WITH_E>
-__device__ __noinline__ float4 box_point_slow(const FFParams &prm, dfl x, dfl y, dfl z, const unsigned short *list, bool wide, int nnear,
+__device__ __noinline__ float4 box_point_slow(const FFParams &prm, dfl x, dfl y, dfl z, const BoxNear &list, bool wide, int nnear,
                                               int ncharged, float4 t, float4 u) {
     for (int j = 0; j < nnear; j++) {
-        const float4 *a = prm.atoms + (size_t)(wide ? reinterpret_cast<const int *>(list)[j] : (int)list[j]) * FF_REC;
+        const float4 *a = prm.atoms + (size_t)list.at(wide, j) * FF_REC;
         const float4 r0 = ldg4(a), r1 = ldg4(a + 1), r2r = ldg4(a + 2);
         const float dx = (x.h + r0.x) + (x.l + r0.z), dy = (y.h + r0.y) + (y.l + r0.w), dz = (z.h + r1.x) + (z.l + r1.y);
         const float dxy2 = fmaf(dx, dx, fmaf(dy, dy, prm.eps));
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(BOX_NT, 2) ff_box_kernel(const __grid_constant
     float4 *tiles = reinterpret_cast<float4 *>(box_raw), *line = tiles;
     float4 *nodes = reinterpret_cast<float4 *>(box_raw + Smem::nodes), *near = nodes;
     __shared__ uint64_t bar[2];
-    __shared__ unsigned short s_near[BOX_NEAR];
+    __shared__ BoxNear s_near;
     __shared__ BoxPick<NT> pk;
     __shared__ dfl s_node[3][N][3];
     __shared__ float s_off[3][N];
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(BOX_NT, 2) ff_box_kernel(const __grid_constant
     for (int k = 0; k < 3; k++) on[k] = df_add(df_add(s_node[0][col / N][k], s_node[1][col % N][k]), s_node[2][0][k]);
     const bool wide = nat > 65536;  // near indices as int
     const int near_cap = wide ? BOX_NEAR / 2 : BOX_NEAR;
-    auto near_at = [&](int i) -> int { return wide ? reinterpret_cast<const int *>(s_near)[i] : (int)s_near[i]; };
+    auto near_at = [&](int i) -> int { return s_near.at(wide, i); };
     int nmid = 0, nzero = 0, place = -1;
     auto pick = [&](const float4 *T, int nj, int want, bool ok) {
         return box_pick<MODE, N, NT>(B, pk, level, nanc, T, nj, want, ok, nmid, nzero, place);
@@ -497,10 +497,7 @@ __global__ void __launch_bounds__(BOX_NT, 2) ff_box_kernel(const __grid_constant
             }
             return;
         }
-        if (place >= 0 && nnear + place < near_cap) {
-            if (wide) reinterpret_cast<int *>(s_near)[nnear + place] = j0;
-            else s_near[nnear + place] = (unsigned short)j0;
-        }
+        if (place >= 0 && nnear + place < near_cap) s_near.set(wide, nnear + place, j0);
         nnear += nzero;
         __syncthreads();
         if (sub < SUBS) {

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
     float4 *tiles = reinterpret_cast<float4 *>(tip_raw);
     dfl *line = reinterpret_cast<dfl *>(tip_raw + Smem::line);    // [K][x][10][10]
     dfl *plane = reinterpret_cast<dfl *>(tip_raw + Smem::plane);  // [K][x - xh][y][10]
-    __shared__ unsigned short s_near[BOX_NEAR];
+    __shared__ BoxNear s_near;
     __shared__ BoxPick<NT> pk;
     __shared__ dfl s_node[3][TIP_N][3], s_pt[3][BOX_S][3];                // parts of the nodes' and the points' positions
     __shared__ dfl s_wx[XS][TIP_N], s_wy[XS][TIP_N], s_wz[XS][TIP_N];
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
     tip_nodes(s_node, tid, p);
     const bool wide = nat > 65536;
     const int near_cap = wide ? BOX_NEAR / 2 : BOX_NEAR;
-    auto near_at = [&](int i) -> int { return wide ? reinterpret_cast<const int *>(s_near)[i] : (int)s_near[i]; };
+    auto near_at = [&](int i) -> int { return s_near.at(wide, i); };
     int nmid = 0, nzero = 0, place = -1, nnear = 0;
     auto gather = [&](int t, bool all) -> int {  // as in ff_box_kernel
         const int i = t * NT + tid;
@@ -401,10 +401,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
         const float4 *T = tiles + (t & 1) * NT * FF_REC;
         const int j0 = gather(t, false);
         box_pick<M_COUL, TIP_N, NT>(B, pk, level, nanc, T, min(NT, ncand - t * NT), 1, true, nmid, nzero, place);
-        if (place >= 0 && nnear + place < near_cap) {
-            if (wide) reinterpret_cast<int *>(s_near)[nnear + place] = j0;
-            else s_near[nnear + place] = (unsigned short)j0;
-        }
+        if (place >= 0 && nnear + place < near_cap) s_near.set(wide, nnear + place, j0);
         nnear += nzero;
         __syncthreads();
         for (int i = on_nodes ? 0 : nmid; i < nmid; i++) {

@@ -109,3 +109,37 @@ def test_tip_boxes_match_float64(gpulib, kind, case):
         if not energy:
             assert (g[:, 3] == (0.25 if accumulate else 0.0)).all()
     assert torch.isfinite(ff.FE).all()
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+def test_tip_boxes_wide_indices(gpulib, kind):
+    """More than 65536 charges, so that boxes list their near ones as 32-bit indices and hand no lists
+    down; most of the charges below the grid, the others a plane in it.  Tolerance as above."""
+    from ppafm_gb300 import device as D
+
+    rng = np.random.default_rng(66000 + kind)
+    n = np.array([113, 112, 97], np.int32)
+    cell = np.diag(n * 0.1)
+    R = np.column_stack([rng.uniform(-8, 19, (66000, 2)), rng.uniform(-60, -14, 66000)])
+    R[-400:, 2] = rng.uniform(0.2, 0.8, 400)  # the highest indices are the near ones
+    q = rng.uniform(-0.3, 0.3, len(R)) * 14.399645
+    atoms, na, nch = D.pack_atoms(R, None, q)
+    ff = D.DeviceFF(n, cell)
+    ff.FE.fill_(float("nan"))
+    got = ff.compute(atoms, na, nch, D.FF_COULOMB, kind=kind, with_E=True).grid4.cpu().numpy().astype(np.float64)
+    assert np.isfinite(got).all()
+    ns = (3, 4, 9)
+    w = 20.0 if kind == 1 else 400.0
+    for i0 in [(0, 0, 0), (50, 61, 3), (17, 90, 40), (110, 108, 88)]:
+        ref = ff.compute_subgrid(i0, ns, atoms, na, nch, D.FF_COULOMB, kind=kind, with_E=True, f64=True).view(-1, 4).cpu().numpy().astype(np.float64)
+        g = got[i0[0] : i0[0] + 3, i0[1] : i0[1] + 4, i0[2] : i0[2] + 9].reshape(-1, 4)
+        P = (np.indices(ns).reshape(3, -1).T + np.array(i0)) * 0.1
+        floor, floor_E = np.zeros(len(P)), np.zeros(len(P))
+        for k, p in enumerate(P):
+            r = np.sqrt(np.maximum(((p - R) ** 2).sum(1), 1e-8))
+            pair = 6 * np.abs(q) / r**3 if kind == 1 else 20 * np.abs(q) / r**4
+            floor[k] = (w * np.abs(q) / r**2).sum() * 2.0**-42 + 1e-9 * pair.sum()
+            floor_E[k] = (w * np.abs(q) / r).sum() * 2.0**-42 + 1e-9 * (pair * r).sum()
+        tol = 2.0**-23 * np.abs(ref) + np.column_stack([floor, floor, floor, floor_E])
+        d = np.abs(g - ref)
+        assert (d <= tol).all(), (i0, float((d / tol).max()))
