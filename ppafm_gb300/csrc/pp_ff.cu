@@ -401,9 +401,9 @@ extern "C" int ppgpu_ff_route(const int *n, const double *cell, const int *ns, i
     FFParams prm;
     int st = ff_params(prm, n, cell, zero, ns, natoms, ncharged, mode, coul_kind, 0.0, 0.0, Qs, QZs, flags);
     if (st) return st;
-    const bool tip = mode == PPGPU_FF_COULOMB && coul_kind != 0;
+    const bool tip = mode == PPGPU_FF_COULOMB && coul_kind != 0, with_e = (flags & PPGPU_FF_WITH_E) != 0;
     FFRoute r = {0, 0};
-    if (!(flags & PPGPU_FF_F64)) r = tip ? ff_tip_route(prm) : ff_box_route(prm, mode, (flags & PPGPU_FF_WITH_E) != 0);
+    if (!(flags & PPGPU_FF_F64)) r = tip ? ff_tip_route(prm, with_e) : ff_box_route(prm, mode, with_e);
     out[0] = r.nodes;
     out[1] = r.levels;
     return set_ok();

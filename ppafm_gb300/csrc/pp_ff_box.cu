@@ -39,26 +39,48 @@ static double tip_reach(const FFParams &prm) {
 // atom-boxes), 128^3, 540 atoms 0.216, 0.224 (2.8e5), 79x251x147, 459 0.335, 0.300 (3.7e5), 320^3, 540 atoms 1.70, 0.79, 0.73 (4.3e6); with 10
 // nodes and 1, 2, 3: 128^3, 540 atoms 0.193, 0.214, 0.232 (2.8e5), slab on 240x240x150 6.6, 4.0, 4.1 (4.2e7), on
 // 320x320x200 11.6, 5.07, 4.95 (9.3e7), on 400x400x250 18.8, 6.8, 5.7 (1.9e8).
+//   Flat and narrow grids: a leaf of few points has no fewer nodes, and nothing can be handed to it that its
+// points have no room for.  1x2000x2000 points, 342 atoms 0.70 against 2.66 ms by boxes, 1x1x20000, 1500 atoms 0.12 against 2.4,
+// 4x400x400, 342 atoms 0.149 against 0.294 with 10 nodes (leaves of 1024 points, 1500 wanted), but 6x400x400, 18540 atoms (LJ)
+// 7.4 against 0.87, 8x200x200, 1500 atoms 0.36 against 0.21.  So the sums have to fit a leaf (10 nodes pay from 1800 points,
+// 8 without anything handed down from 1024), and leaves below 2000 points take as many more atoms.
+//   Few boxes whose reach is long: nearly all atoms are near ones, unless they fill much more space than that.  51x32x136 points at
+// 0.34 A, solid of 3869 atoms 0.58 against 1.38 ms, 55x144x27 at 0.4 A, slab of 1967 0.30 against 0.55; but 18540 atoms of
+// the slab on 101x101x63 at 0.4 A 5.5 against 2.8.  Below 240 boxes and beyond 14 A: atoms as many as the reach cubed.
+//   10 nodes for their shorter reach alone: 23x188x258 at 0.47 A, 63 atoms 0.093 against 0.136, 22x15x2322 at 0.4 A, 234 atoms
+// 0.095 against 0.192, 192x194x178 at 0.47, 297 atoms 1.05 against 0.28: half as many atoms again.
+//   Of 3370 calls of plausible molecules, layers, slabs and solids (16 to 300 points an axis, half of them flat or narrow, 0.05 to 0.6
+// A) 39 are slower by boxes than pair by pair, by 1.2 times in the mean.
 struct BoxChoice {
     int N, levels;
     bool boxes;
 };
 static BoxChoice box_choice(const FFParams &prm, int mode, bool with_e, BoxPrm *B) {
     const double reach = tip_reach(prm), nat = mode == M_COUL ? prm.ncharged : prm.natoms;
+    const int NC = (with_e ? 4 : 3) * (mode == M_LJC ? 2 : 1);  // sums of a node
     BoxChoice c;
     double H;
     box_plan(prm, 8, box_kappa(8, mode), reach, B, &H);
     const double boxes = (double)B->nb[0] * B->nb[1] * B->nb[2], work = nat * boxes;
-    const bool dense = mode == M_LJC && with_e ? nat >= 2.0 * boxes : nat >= 1.2 * boxes || (nat >= 0.45 * boxes && (work >= 1.1e5 || H * box_kappa(8, mode) >= 12.0));
-    c.N = !prm.accumulate && (dense || H * box_kappa(8, mode) > 36.0) ? 10 : 8;
-    if (c.N == 10) box_plan(prm, 10, box_kappa(10, mode), reach, B, &H);
+    const double far8 = H * box_kappa(8, mode);
+    const bool dense = mode == M_LJC && with_e ? nat >= 2.0 * boxes : nat >= 1.2 * boxes || (nat >= 0.45 * boxes && (work >= 1.1e5 || far8 >= 12.0));
+    c.N = 8;
+    if (!prm.accumulate && (dense || far8 > 36.0)) {
+        box_plan(prm, 10, box_kappa(10, mode), reach, B, &H);
+        if (box_leaf(*B) >= std::max(1800, 250 * NC)) c.N = 10;
+        else box_plan(prm, 8, box_kappa(8, mode), reach, B, &H);
+    }
     if (c.N == 8) c.levels = work < 3e5 ? 0 : (work < 3e6 ? 1 : (work < 1e9 ? 2 : 3));
     else c.levels = work < 8e6 ? 1 : (work < 8e7 ? 2 : 3);
     B->levels = prm.accumulate ? 0 : c.levels;
     const double pairs = nat + (mode == M_QZS && prm.nqa > 0 ? 4.0 * prm.ncharged : 0.0);
-    const double far = H * box_kappa(c.N, mode);
-    if (boxes >= 304) c.boxes = far <= 36.0 && pairs >= 40.0 + 20480.0 / boxes;
-    else c.boxes = boxes >= 64 && far <= 24.0 && pairs >= 40.0 + (boxes >= 200 ? 51200.0 : 70000.0) / boxes;
+    const double far = H * box_kappa(c.N, mode), leaf = box_leaf(*B);
+    double need = 40.0 + (boxes >= 304 ? 20480.0 : (boxes >= 200 ? 51200.0 : 70000.0)) / boxes;
+    if (leaf < 2000.0) need *= 2000.0 / leaf;
+    if (c.N == 10 && !dense) need *= 1.5;
+    c.boxes = boxes >= 64 && pairs >= need && far <= (boxes >= 304 ? 36.0 : 24.0);
+    if (c.N == 8 && leaf < (B->levels == 0 ? 1024 : 128 * NC)) c.boxes = false;
+    if (boxes < 240 && far > 14.0 && pairs < far * far * far) c.boxes = false;
     return c;
 }
 

@@ -433,6 +433,9 @@ static inline void box_plan(const FFParams &prm, int N, double kappa, double rea
     }
 }
 
+// Points of a leaf (a smaller one where their sizes differ).
+static inline int box_leaf(const BoxPrm &B) { return B.s[0] * B.s[1] * B.s[2]; }
+
 // CTAs of a cluster for each of n upper boxes: enough to fill the SMs (two CTAs each).
 static inline int box_cluster(long long n) {
     int c = 1;

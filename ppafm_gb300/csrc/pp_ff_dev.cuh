@@ -57,7 +57,7 @@ struct FFRoute {
     int nodes, levels;
 };
 FFRoute ff_box_route(const FFParams &prm, int mode, bool with_e);
-FFRoute ff_tip_route(const FFParams &prm);
+FFRoute ff_tip_route(const FFParams &prm, bool with_e);
 // The pz (1) and dz2 (2) Coulomb tips in double-float (pp_ff_tip.cu).
 int launch_ff_tip(FFParams &prm, int kind, bool with_e, bool ortho, cudaStream_t st);
 

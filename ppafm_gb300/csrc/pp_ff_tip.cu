@@ -558,17 +558,21 @@ static int launch_tip_boxes(const FFParams &prm, BoxPrm B, cudaStream_t st) {
 // 64^3 (64 leaves) 342: 0.69 against 0.83, the boxes too few for 152 SMs.
 //   Levels above the leaves, 0, 1 and 2: 140^3, 90 charges 0.92, 0.94, 0.98 ms (6.6e4 charge-boxes), 96^3, 342 1.22, 1.03,
 // 1.06 (7.4e4), 140^3, 540 3.69, 1.94, 1.99 (3.9e5), 200^3, 342 6.6, 2.15, 1.86 (7.5e5).
-static bool tip_box_rule(const FFParams &prm, double H, BoxPrm *B) {
-    const double boxes = (double)B->nb[0] * B->nb[1] * B->nb[2], work = prm.ncharged * boxes;
+//   Flat and narrow grids, whose leaves have few points for the 1000 nodes, or no room for what is handed to them (pair by
+// pair against by boxes): 990x1x547, 138 charges 0.39 against 3.1 ms, 2x319x1251, 567 2.5 against 9.0, 4x613x123, 585 1.35 against
+// 3.1.  Of 900 calls (half of them flat or narrow) 3 are slower by boxes than pair by pair, by 1.3 times.
+static bool tip_box_rule(const FFParams &prm, bool with_e, double H, BoxPrm *B) {
+    const double boxes = (double)B->nb[0] * B->nb[1] * B->nb[2], work = prm.ncharged * boxes, leaf = box_leaf(*B);
     B->levels = prm.accumulate || work < 7e4 ? 0 : (work < 5e5 ? 1 : (work < 1e8 ? 2 : 3));
-    return boxes >= 200 && H * TIP_KAPPA <= 36.0 && prm.ncharged >= 15.0 + 20000.0 / boxes;
+    if (leaf < (B->levels == 0 ? 1024 : (with_e ? 2000 : 1500))) return false;
+    return boxes >= 200 && H * TIP_KAPPA <= 36.0 && prm.ncharged >= (15.0 + 20000.0 / boxes) * std::max(1.0, 2500.0 / leaf);
 }
 
-FFRoute ff_tip_route(const FFParams &prm) {
+FFRoute ff_tip_route(const FFParams &prm, bool with_e) {
     BoxPrm B;
     double H;
     box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, &B, &H);
-    return tip_box_rule(prm, H, &B) ? FFRoute{TIP_N, B.levels} : FFRoute{0, 0};
+    return tip_box_rule(prm, with_e, H, &B) ? FFRoute{TIP_N, B.levels} : FFRoute{0, 0};
 }
 
 template <int KIND, bool WITH_E, bool ORTHO>
@@ -576,7 +580,7 @@ static int launch_tip(FFParams &prm, cudaStream_t st) {
     BoxPrm B;
     double H;
     box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, &B, &H);
-    if (tip_box_rule(prm, H, &B)) return launch_tip_boxes<KIND, WITH_E, ORTHO>(prm, B, st);
+    if (tip_box_rule(prm, WITH_E, H, &B)) return launch_tip_boxes<KIND, WITH_E, ORTHO>(prm, B, st);
     prm.nzc = (prm.ns[2] + TIP_P - 1) / TIP_P;
     prm.nchunks = (long long)prm.ns[0] * prm.ns[1] * prm.nzc;
     const long long nblk = (prm.nchunks + TIP_THREADS - 1) / TIP_THREADS;

@@ -84,3 +84,31 @@ def test_routes_of_small_and_float64_calls(route):
     assert route((200, 200, 200), 0.1, 342, 342, LJC, flags=F64) == (0, 0)
     assert route((200, 200, 200), 0.1, 0, 0, LJC) == (0, 0)
     assert route((200, 200, 200), 0.1, 342, 342, LJC, ns=(0, 200, 200)) == (0, 0)
+
+
+@pytest.mark.parametrize("mode", [LJ, COULOMB, LJC, QZS])
+@pytest.mark.parametrize("n", [(1, 2000, 2000), (2000, 1, 2000), (1, 1, 20000), (2, 1, 20000), (1500, 1, 400), (1, 300, 300)])
+def test_planes_and_lines_go_pair_by_pair(route, mode, n):
+    """Their leaves have fewer points than a box has nodes: by boxes they took 3 to 20 times as long."""
+    for natoms in (60, 342, 1500, 18540):
+        for flags in (0, WITH_E, ACCUMULATE):
+            assert route(n, 0.1, natoms, natoms, mode, flags=flags) == (0, 0)
+            assert route(n, 0.1, natoms, natoms, COULOMB, kind=2, flags=flags) == (0, 0)
+    # a plane of a grid that itself goes by boxes
+    assert route((200, 200, 200), 0.1, 342, 342, mode, ns=(1, 200, 200)) == (0, 0)
+
+
+@pytest.mark.parametrize(
+    "n,step,natoms,mode,want",
+    [
+        ((6, 400, 400), 0.1, 18540, LJ, (8, 2)),  # leaves of 1536 points
+        ((4, 400, 400), 0.1, 1500, LJC, (8, 1)),  # 1024 points: no room for 6 x 250 cells of 10 nodes
+        ((2, 400, 400), 0.1, 1500, LJC, (0, 0)),  # 512 points: nor of 8
+        ((51, 32, 136), 0.335, 3869, LJC, (0, 0)),  # few boxes, most atoms within their reach
+        ((101, 101, 63), 0.396, 18540, LJC, (10, 1)),  # few boxes, atoms far beyond it
+        ((23, 188, 258), 0.468, 63, LJC, (0, 0)),  # 10 nodes for their shorter reach: few atoms
+        ((192, 194, 178), 0.47, 297, LJC, (10, 1)),
+    ],
+)
+def test_route_by_points_boxes_and_reach(route, n, step, natoms, mode, want):
+    assert route(n, step, natoms, natoms if mode != LJ else 0, mode) == want
