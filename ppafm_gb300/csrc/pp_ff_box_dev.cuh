@@ -218,14 +218,21 @@ __device__ __forceinline__ unsigned short *share_list(const BoxShare &s, int i) 
 // rounded operations, because the CTAs of several levels have to agree on it.  rep: the interpolation
 // error of the r^-13 force at kappa H (5e-6 of the term with 8 nodes at 7, 2e-5 with 10 at 4.25) over
 // the 1.5e-7 allowed of the r^-7 force, times (kappa H)^N, with whose power over r it falls.
+//   No distance would be enough for an atom without attraction.  Where the r^-13 force is the larger
+// one, the error is held against it instead, beyond 1.55 (8 nodes) or 1.63 (10) kappa H.  18540 atoms with c6 = 0 on 200^3
+// points: 82 ms with all of them near, 7.2 now, 53 pair by pair; error against 64 bits 2.5e-7, 3.8e-7, 4.1e-7.
 template <int MODE, int N>
 __device__ __forceinline__ bool box_far(const float4 &r0, const float4 &r1, const float4 &c, float far2, float rep) {
     const float dx = __fadd_rn(c.x, r0.x), dy = __fadd_rn(c.y, r0.y), dz = __fadd_rn(c.z, r1.x);
     const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
     if (!(r2 >= far2)) return false;
     if (MODE == M_COUL) return true;
-    const float r4 = __fmul_rn(r2, r2), r8 = __fmul_rn(r4, r4), rn = __fmul_rn(r8, N == 8 ? __fmul_rn(r4, r2) : r8);  // r^(6 + N)
-    return __fmul_rn(fabsf(r1.w), rep) <= __fmul_rn(fabsf(r1.z), fminf(rn, 3e38f));
+    const float c6 = fabsf(r1.z), c12 = fabsf(r1.w);
+    const float r4 = __fmul_rn(r2, r2), r8 = __fmul_rn(r4, r4), r6 = __fmul_rn(r4, r2);
+    const float rn = N == 8 ? __fmul_rn(r8, r6) : __fmul_rn(r8, r8);  // r^(6 + N)
+    if (__fmul_rn(c12, rep) <= __fmul_rn(c6, fminf(rn, 3e38f))) return true;
+    const float rN = N == 8 ? r8 : __fmul_rn(r8, r2);
+    return rN >= rep && __fmul_rn(c6, r6) <= c12 && c12 <= 3e38f;
 }
 
 // A CTA's box at a level and its points; boxes are numbered along z first.

@@ -125,6 +125,57 @@ def test_more_boxes_match_float64(gpulib, case):
     test_boxes_match_float64(gpulib, case)
 
 
+REPULSIVE = [
+    ("lj", (130, 129, 113), 0.1, False, 200, "plane", 1.0, True, False),  # 8 nodes
+    ("ljc", (113, 129, 97), 0.1, True, 260, "plane", 0.5, False, True),
+    ("lj", (160, 113, 128), 0.1, False, 3000, "slab", 1.0, False, False),  # 10 nodes and levels
+    ("ljc", (113, 129, 97), 0.1, False, 1300, "slab", 0.7, True, False),
+]
+
+
+@pytest.mark.parametrize("share", [0.5, 1.0])
+@pytest.mark.parametrize("case", REPULSIVE, ids=lambda c: "-".join(map(str, (c[0], *c[1], c[4], c[5]))))
+def test_atoms_without_attraction(gpulib, monkeypatch, case, share):
+    """c6 = 0 for a share of the atoms: far from a distance at which the r^-13 force itself is
+    interpolated to 1.5e-7.  Same tolerance."""
+    import sys
+
+    whole = _atoms
+
+    def some(rng, natoms, cell, kind):
+        R, c, q = whole(rng, natoms, cell, kind)
+        c[: int(share * natoms), 0] = 0.0
+        return R, c, q
+
+    monkeypatch.setattr(sys.modules[__name__], "_atoms", some)
+    test_boxes_match_float64(gpulib, case)
+
+
+def test_atoms_without_attraction_are_far(gpulib):
+    """They are left to the nodes like others: the field of 18540 of them takes a few times that of
+    attractive ones (all near, it took 30 times as long and longer than pair by pair)."""
+    import torch
+
+    from ppafm_gb300 import device as D
+
+    n, cell = (200, 200, 200), np.diag([20.0, 20.0, 20.0])
+    R, c, _ = _atoms(np.random.default_rng(4), 18540, cell, "slab")
+    ff = D.DeviceFF(n, cell)
+    ms = []
+    for c6 in (1.0, 0.0):
+        rec, na, _ = D.pack_atoms(R, c * [c6, 1.0], None)
+        t = []
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            ff.compute(rec, na, 0, D.FF_LJ)
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+        ms.append(min(t))
+    assert ms[1] < 8.0 * ms[0], ms
+
+
 def _subgrid_f64(ff, i0, ns, rec, na, nch, mode, Q, Fmax, flags, tip):
     """A sub-box of the grid in float64 (compute_subgrid has no tip charges)."""
     import torch
