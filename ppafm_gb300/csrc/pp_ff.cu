@@ -249,8 +249,8 @@ static int launch_ff_e(FFParams &prm, bool with_e, bool ortho, cudaStream_t st) 
 }
 
 static int ff_dispatch(FFParams &prm, int mode, int kind, bool with_e, bool ortho, cudaStream_t st) {
-    if (!(mode == PPGPU_FF_COULOMB && kind != 0) && ff_box_rule(prm, mode, with_e))
-        return launch_ff_box(prm, mode, with_e, ortho, st);
+    int rc;
+    if (!(mode == PPGPU_FF_COULOMB && kind != 0) && launch_ff_box(prm, mode, with_e, ortho, st, &rc)) return rc;
     switch (mode) {
         case PPGPU_FF_LJ:
             return launch_ff_e<M_LJ, 4>(prm, with_e, ortho, st);

@@ -56,15 +56,17 @@ struct BoxChoice {
     bool boxes;
 };
 static BoxChoice box_choice(const FFParams &prm, int mode, bool with_e, BoxPrm *B) {
-    const double reach = tip_reach(prm), nat = mode == M_COUL ? prm.ncharged : prm.natoms;
+    const double nat = mode == M_COUL ? prm.ncharged : prm.natoms, boxes = box_count(prm), work = nat * boxes;
+    const double pairs = nat + (mode == M_QZS && prm.nqa > 0 ? 4.0 * prm.ncharged : 0.0);
+    double need = 40.0 + (boxes >= 304 ? 20480.0 : (boxes >= 200 ? 51200.0 : 70000.0)) / boxes;
+    BoxChoice c = {8, 0, false};
+    if (!(boxes >= 64 && pairs >= need)) return c;  // small calls: planning takes a third of a microsecond
+    const double reach = tip_reach(prm);
     const int NC = (with_e ? 4 : 3) * (mode == M_LJC ? 2 : 1);  // sums of a node
-    BoxChoice c;
     double H;
     box_plan(prm, 8, box_kappa(8, mode), reach, B, &H);
-    const double boxes = (double)B->nb[0] * B->nb[1] * B->nb[2], work = nat * boxes;
     const double far8 = H * box_kappa(8, mode);
     const bool dense = mode == M_LJC && with_e ? nat >= 2.0 * boxes : nat >= 1.2 * boxes || (nat >= 0.45 * boxes && (work >= 1.1e5 || far8 >= 12.0));
-    c.N = 8;
     if (!prm.accumulate && (dense || far8 > 36.0)) {
         box_plan(prm, 10, box_kappa(10, mode), reach, B, &H);
         if (box_leaf(*B) >= std::max(1800, 250 * NC)) c.N = 10;
@@ -73,20 +75,13 @@ static BoxChoice box_choice(const FFParams &prm, int mode, bool with_e, BoxPrm *
     if (c.N == 8) c.levels = work < 3e5 ? 0 : (work < 3e6 ? 1 : (work < 1e9 ? 2 : 3));
     else c.levels = work < 8e6 ? 1 : (work < 8e7 ? 2 : 3);
     B->levels = prm.accumulate ? 0 : c.levels;
-    const double pairs = nat + (mode == M_QZS && prm.nqa > 0 ? 4.0 * prm.ncharged : 0.0);
     const double far = H * box_kappa(c.N, mode), leaf = box_leaf(*B);
-    double need = 40.0 + (boxes >= 304 ? 20480.0 : (boxes >= 200 ? 51200.0 : 70000.0)) / boxes;
     if (leaf < 2000.0) need *= 2000.0 / leaf;
     if (c.N == 10 && !dense) need *= 1.5;
-    c.boxes = boxes >= 64 && pairs >= need && far <= (boxes >= 304 ? 36.0 : 24.0);
+    c.boxes = pairs >= need && far <= (boxes >= 304 ? 36.0 : 24.0);
     if (c.N == 8 && leaf < (B->levels == 0 ? 1024 : 128 * NC)) c.boxes = false;
     if (boxes < 240 && far > 14.0 && pairs < far * far * far) c.boxes = false;
     return c;
-}
-
-bool ff_box_rule(const FFParams &prm, int mode, bool with_e) {
-    BoxPrm B;
-    return box_choice(prm, mode, with_e, &B).boxes;
 }
 
 FFRoute ff_box_route(const FFParams &prm, int mode, bool with_e) {
@@ -95,9 +90,12 @@ FFRoute ff_box_route(const FFParams &prm, int mode, bool with_e) {
     return c.boxes ? FFRoute{c.N, B.levels} : FFRoute{0, 0};
 }
 
-int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st) {
+bool launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st, int *rc) {
     BoxPrm B;
-    return box_choice(prm, mode, with_e, &B).N == 8 ? launch_box_nodes<8>(prm, B, mode, with_e, ortho, st) : launch_ff_box10(prm, B, mode, with_e, ortho, st);
+    const BoxChoice c = box_choice(prm, mode, with_e, &B);
+    if (!c.boxes) return false;
+    *rc = c.N == 8 ? launch_box_nodes<8>(prm, B, mode, with_e, ortho, st) : launch_ff_box10(prm, B, mode, with_e, ortho, st);
+    return true;
 }
 
 }  // namespace ppgpu

@@ -391,6 +391,13 @@ __device__ __forceinline__ void async_wait() {
 
 // ------------------------------------------------------------------------------ host
 
+// Leaves of a grid.
+static inline double box_count(const FFParams &prm) {
+    double n = 1.0;
+    for (int k = 0; k < 3; k++) n *= (prm.ns[k] + BOX_S - 1) / BOX_S;
+    return n;
+}
+
 // The leaves of a grid and the levels above them; half0: H of a leaf.  Far at a level: kappa H, and
 // the reach of the tip's charges.  H is the half diagonal, or that of a cube of the longest
 // edge: the error follows the nearest singularity beside the longest edge, and kappa is a cube's.

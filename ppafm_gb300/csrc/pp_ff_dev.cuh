@@ -49,9 +49,9 @@ inline void ff_set_offsets(FFParams &prm) {
         for (int i = 0; i < FF_MAX_P; i++) prm.off[c][i] = (float)(prm.dC[c] * i);
 }
 
-// Force fields by boxes (pp_ff_box.cu): whether a grid and its atoms are summed that way.
-bool ff_box_rule(const FFParams &prm, int mode, bool with_e);
-int launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st);
+// Force fields by boxes (pp_ff_box.cu): sums a grid and its atoms that way and sets the status, or
+// leaves them (false) where pair by pair is the faster.
+bool launch_ff_box(const FFParams &prm, int mode, bool with_e, bool ortho, cudaStream_t st, int *rc);
 // Nodes per axis of its boxes (0: pair by pair) and levels of boxes above the leaves.
 struct FFRoute {
     int nodes, levels;

@@ -561,26 +561,26 @@ static int launch_tip_boxes(const FFParams &prm, BoxPrm B, cudaStream_t st) {
 //   Flat and narrow grids, whose leaves have few points for the 1000 nodes, or no room for what is handed to them (pair by
 // pair against by boxes): 990x1x547, 138 charges 0.39 against 3.1 ms, 2x319x1251, 567 2.5 against 9.0, 4x613x123, 585 1.35 against
 // 3.1.  Of 900 calls (half of them flat or narrow) 3 are slower by boxes than pair by pair, by 1.3 times.
-static bool tip_box_rule(const FFParams &prm, bool with_e, double H, BoxPrm *B) {
-    const double boxes = (double)B->nb[0] * B->nb[1] * B->nb[2], work = prm.ncharged * boxes, leaf = box_leaf(*B);
+static bool tip_box_rule(const FFParams &prm, bool with_e, BoxPrm *B) {
+    const double boxes = box_count(prm), work = prm.ncharged * boxes, need = 15.0 + 20000.0 / boxes;
+    if (!(boxes >= 200 && prm.ncharged >= need)) return false;  // before planning, which small calls would feel
+    double H;
+    box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, B, &H);
     B->levels = prm.accumulate || work < 7e4 ? 0 : (work < 5e5 ? 1 : (work < 1e8 ? 2 : 3));
+    const double leaf = box_leaf(*B);
     if (leaf < (B->levels == 0 ? 1024 : (with_e ? 2000 : 1500))) return false;
-    return boxes >= 200 && H * TIP_KAPPA <= 36.0 && prm.ncharged >= (15.0 + 20000.0 / boxes) * std::max(1.0, 2500.0 / leaf);
+    return H * TIP_KAPPA <= 36.0 && prm.ncharged >= need * std::max(1.0, 2500.0 / leaf);
 }
 
 FFRoute ff_tip_route(const FFParams &prm, bool with_e) {
     BoxPrm B;
-    double H;
-    box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, &B, &H);
-    return tip_box_rule(prm, with_e, H, &B) ? FFRoute{TIP_N, B.levels} : FFRoute{0, 0};
+    return tip_box_rule(prm, with_e, &B) ? FFRoute{TIP_N, B.levels} : FFRoute{0, 0};
 }
 
 template <int KIND, bool WITH_E, bool ORTHO>
 static int launch_tip(FFParams &prm, cudaStream_t st) {
     BoxPrm B;
-    double H;
-    box_plan(prm, TIP_N, TIP_KAPPA, TIP_H, &B, &H);
-    if (tip_box_rule(prm, WITH_E, H, &B)) return launch_tip_boxes<KIND, WITH_E, ORTHO>(prm, B, st);
+    if (tip_box_rule(prm, WITH_E, &B)) return launch_tip_boxes<KIND, WITH_E, ORTHO>(prm, B, st);
     prm.nzc = (prm.ns[2] + TIP_P - 1) / TIP_P;
     prm.nchunks = (long long)prm.ns[0] * prm.ns[1] * prm.nzc;
     const long long nblk = (prm.nchunks + TIP_THREADS - 1) / TIP_THREADS;
