@@ -12,8 +12,8 @@
 // Design (GB300):
 //  * One lane per stroke (pixel column), or one per axis of a stroke on scans too small to fill
 //    the GPU (relax_axis_kernel).  A lane's whole z-walk is a single flattened loop in which
-//    every trip interpolates the force once (8 x 16-byte __ldg of the interleaved float4 grid,
-//    when the probe has left its cell), so lanes that converge early at one height move on to
+//    every trip interpolates the force once (8 x 16-byte __ldg of the interleaved float4 grid;
+//    scans of one wave only when the probe has left its cell), so lanes that converge early at one height move on to
 //    their next height instead of idling; the warp leaves the loop on a vote once all of its
 //    lanes have finished their strokes.
 //  * Precision, chosen by measurement against the float64 reference on a GB300, whose
@@ -64,28 +64,43 @@ struct Corners4 {
     float4 c[8];
 };
 
-// Same, all four channels, at a float grid coordinate (AFMulator path).
+// The same as interp_force_df, all four channels, at a float grid coordinate (AFMulator path); KEEP:
+// gathering when the stroke has left its cell.
+template <bool KEEP>
 __device__ __forceinline__ float4 interp_fe4(const float4 *__restrict__ FE, int n0, int n1, int n2, float3 g, Corners4 &K) {
     const float fx = floorf(g.x), fy = floorf(g.y), fz = floorf(g.z);
     const float tx = g.x - fx, ty = g.y - fy, tz = g.z - fz;
     const float mx = 1.f - tx, my = 1.f - ty, mz = 1.f - tz;
     const int ix0 = wrap_index((int)fx, n0), iy0 = wrap_index((int)fy, n1), iz0 = wrap_index((int)fz, n2);
-    const long long cell = ((long long)ix0 * n1 + iy0) * n2 + iz0;
-    if (cell != K.cell) {
-        K.cell = cell;
-        const long long dx = ix0 + 1 == n0 ? -(long long)ix0 * n1 * n2 : (long long)n1 * n2;
-        const long long dy = iy0 + 1 == n1 ? -(long long)iy0 * n2 : (long long)n2;
-        const int dz = iz0 + 1 == n2 ? -iz0 : 1;
+    float4 *c = K.c;
+    if (!KEEP) {
+        const int ix1 = (ix0 + 1 == n0) ? 0 : ix0 + 1;
+        const int iy1 = (iy0 + 1 == n1) ? 0 : iy0 + 1;
+        const int iz1 = (iz0 + 1 == n2) ? 0 : iz0 + 1;
+        const long long r00 = ((long long)ix0 * n1 + iy0) * n2, r01 = ((long long)ix0 * n1 + iy1) * n2;
+        const long long r10 = ((long long)ix1 * n1 + iy0) * n2, r11 = ((long long)ix1 * n1 + iy1) * n2;
+        c[0] = ldg4(FE + r00 + iz0), c[1] = ldg4(FE + r00 + iz1);
+        c[2] = ldg4(FE + r01 + iz0), c[3] = ldg4(FE + r01 + iz1);
+        c[4] = ldg4(FE + r10 + iz0), c[5] = ldg4(FE + r10 + iz1);
+        c[6] = ldg4(FE + r11 + iz0), c[7] = ldg4(FE + r11 + iz1);
+    } else {
+        const long long cell = ((long long)ix0 * n1 + iy0) * n2 + iz0;
+        if (cell != K.cell) {
+            K.cell = cell;
+            const long long dx = ix0 + 1 == n0 ? -(long long)ix0 * n1 * n2 : (long long)n1 * n2;
+            const long long dy = iy0 + 1 == n1 ? -(long long)iy0 * n2 : (long long)n2;
+            const int dz = iz0 + 1 == n2 ? -iz0 : 1;
 #pragma unroll
-        for (int k = 0; k < 8; k++) K.c[k] = ldg4(FE + cell + ((k & 4) ? dx : 0) + ((k & 2) ? dy : 0) + ((k & 1) ? dz : 0));
+            for (int k = 0; k < 8; k++) c[k] = ldg4(FE + cell + ((k & 4) ? dx : 0) + ((k & 2) ? dy : 0) + ((k & 1) ? dz : 0));
+        }
     }
     float4 o;
-#define PP_LERP3(a)                                                                                    \
-    {                                                                                                  \
-        const float v00 = fmaf(K.c[4].a, tx, K.c[0].a * mx), v10 = fmaf(K.c[6].a, tx, K.c[2].a * mx); \
-        const float v01 = fmaf(K.c[5].a, tx, K.c[1].a * mx), v11 = fmaf(K.c[7].a, tx, K.c[3].a * mx); \
-        const float v0 = fmaf(v10, ty, v00 * my), v1 = fmaf(v11, ty, v01 * my);                       \
-        o.a = fmaf(v1, tz, v0 * mz);                                                                   \
+#define PP_LERP3(a)                                                                                \
+    {                                                                                              \
+        const float v00 = fmaf(c[4].a, tx, c[0].a * mx), v10 = fmaf(c[6].a, tx, c[2].a * mx);     \
+        const float v01 = fmaf(c[5].a, tx, c[1].a * mx), v11 = fmaf(c[7].a, tx, c[3].a * mx);     \
+        const float v0 = fmaf(v10, ty, v00 * my), v1 = fmaf(v11, ty, v01 * my);                   \
+        o.a = fmaf(v1, tz, v0 * mz);                                                               \
     }
     PP_LERP3(x) PP_LERP3(y) PP_LERP3(z) PP_LERP3(w)
 #undef PP_LERP3
@@ -119,8 +134,9 @@ __device__ __forceinline__ void fill_ztab(dfl *ztab, const RelaxPrm &P, const do
 // TPS lanes per stroke (1, 2, 4 or 8): the lanes of a group hold the same state and split
 // each trilinear gather (interp_force_df_group, bit-identical to one lane); lane 0 of the
 // group writes the outputs.  More lanes per stroke put more warps in flight when a scan has
-// few strokes, which is what bounds this kernel.
-template <bool SCAN, int TPS, bool SPL>
+// few strokes, which is what bounds this kernel.  KEEP (one lane): the corner values of the
+// stroke's cell are kept until it leaves it.
+template <bool SCAN, int TPS, bool SPL, bool KEEP>
 __global__ void __launch_bounds__(RELAX_THREADS) relax_kernel(const RelaxPrm P, const StrokeIO S, const ScanIO C) {
     extern __shared__ dfl ztab[];
     const int s = (blockIdx.x * RELAX_THREADS + threadIdx.x) / TPS;
@@ -180,14 +196,15 @@ __global__ void __launch_bounds__(RELAX_THREADS) relax_kernel(const RelaxPrm P, 
         set_height(0);
     }
 
-    Corners corners;
+    Corners corners;  // KEEP
     corners.cell = -1;
     unsigned am;
     while ((am = __ballot_sync(FULL, active)) != 0u) {
         if (!active) continue;
         dfl u[3], F[3];
         grid_coord_df(P.dic, P.diag, tf, d, u);
-        interp_force_df_group<TPS>(P.FE, P.n0, P.n1, P.n2, base, u, F, sub, am, corners);
+        if constexpr (KEEP) interp_force_df(P.FE, P.n0, P.n1, P.n2, base, u, F, corners);
+        else interp_force_df_group<TPS>(P.FE, P.n0, P.n1, P.n2, base, u, F, sub, am);
         if (fin) {
             // outputs of height iz: position after the last move, grid force there
             dfl r[3];
@@ -497,6 +514,7 @@ __device__ __forceinline__ float dot3(float3 a, const float *b) { return a.x * b
 
 constexpr int AFM_RELAX_THREADS = 128;  // as the single-grid kernel: packs beside the next image's force field
 
+template <bool KEEP>
 __global__ void __launch_bounds__(AFM_RELAX_THREADS) relax_afm_kernel(const AfmPrm P) {
     const int p = blockIdx.x * AFM_RELAX_THREADS + threadIdx.x;
     bool active = p < P.npix && P.nz > 0;
@@ -525,7 +543,7 @@ __global__ void __launch_bounds__(AFM_RELAX_THREADS) relax_afm_kernel(const AfmP
         g.x = dot3(pos, P.dic);
         g.y = dot3(pos, P.dic + 3);
         g.z = dot3(pos, P.dic + 6);
-        const float4 fe = interp_fe4(P.FE, P.n0, P.n1, P.n2, g, corners);
+        const float4 fe = interp_fe4<KEEP>(P.FE, P.n0, P.n1, P.n2, g, corners);
         float3 f = make_float3(fe.x, fe.y, fe.z);
         const float3 dp = make_float3(pos.x - tip.x, pos.y - tip.y, pos.z - tip.z);
         const float3 dq = make_float3(dot3(dp, P.tA), dot3(dp, P.tB), dot3(dp, P.tC));
@@ -792,14 +810,25 @@ static int g_relax_tps = 0;  // 0: the default
 
 static int relax_tps(long long) { return g_relax_tps ? g_relax_tps : 1; }
 
+// Strokes keep the corners of their cell (Corners, Corners4) while all of them fit the GPU at once: the
+// registers cost a CTA a SM (122 instead of 96: 4 instead of 5; the AFMulator's 79 instead of 56: 6
+// instead of 9), which a scan of one wave does not miss and a larger one does.  One lane, 30 heights, every trip
+// gathered against corners kept, ms: 180^2 strokes 1.21, 1.17, 260^2 (67 600) 1.82, 1.78, but 300^2 2.24, 2.36, 420^2 4.09, 4.14; with a
+// tip spline 260^2 2.30, 2.26, 300^2 2.78, 3.17, 512^2 7.13, 7.47; on a tilted cell 260^2 2.04, 2.02, 300^2 2.50, 2.63.
+// AFMulator: 256^2 1.01, 0.94, 340^2 (115 600) 1.25, 1.17, 400^2 1.61, 1.63, 640^2 3.27, 3.38.
+constexpr long long KEEP_MAX_STROKES = 4LL * 152 * RELAX_THREADS;
+constexpr long long AFM_KEEP_MAX_STROKES = 6LL * 152 * AFM_RELAX_THREADS;
+
 template <bool SCAN, bool SPL>
-static void launch_relax_t(int tps, unsigned nblk, size_t smem, cudaStream_t st, const RelaxPrm &P, const StrokeIO &S,
+static void launch_relax_t(int tps, bool keep, unsigned nblk, size_t smem, cudaStream_t st, const RelaxPrm &P, const StrokeIO &S,
                            const ScanIO &C) {
     switch (tps) {
-    case 8: relax_kernel<SCAN, 8, SPL><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
-    case 4: relax_kernel<SCAN, 4, SPL><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
-    case 2: relax_kernel<SCAN, 2, SPL><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
-    default: relax_kernel<SCAN, 1, SPL><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
+    case 8: relax_kernel<SCAN, 8, SPL, false><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
+    case 4: relax_kernel<SCAN, 4, SPL, false><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
+    case 2: relax_kernel<SCAN, 2, SPL, false><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C); break;
+    default:
+        if (keep) relax_kernel<SCAN, 1, SPL, true><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C);
+        else relax_kernel<SCAN, 1, SPL, false><<<nblk, RELAX_THREADS, smem, st>>>(P, S, C);
     }
 }
 
@@ -813,10 +842,11 @@ static void launch_relax(int tps, long long nstroke, size_t smem, cudaStream_t s
         return;
     }
     const unsigned nblk = (unsigned)((nstroke * tps + RELAX_THREADS - 1) / RELAX_THREADS);
+    const bool keep = nstroke <= KEEP_MAX_STROKES;
     if (P.spl.n > 0)
-        launch_relax_t<SCAN, true>(tps, nblk, smem, st, P, S, C);
+        launch_relax_t<SCAN, true>(tps, keep, nblk, smem, st, P, S, C);
     else
-        launch_relax_t<SCAN, false>(tps, nblk, smem, st, P, S, C);
+        launch_relax_t<SCAN, false>(tps, keep, nblk, smem, st, P, S, C);
 }
 
 }  // namespace ppgpu
@@ -947,7 +977,8 @@ extern "C" int ppgpu_relax_afm(const float *FE, const int *n, const double *inv_
         return set_ok();
     }
     const unsigned nblk = (unsigned)((npix + AFM_RELAX_THREADS - 1) / AFM_RELAX_THREADS);
-    relax_afm_kernel<<<nblk, AFM_RELAX_THREADS, 0, (cudaStream_t)stream>>>(P);
+    if (npix <= AFM_KEEP_MAX_STROKES) relax_afm_kernel<true><<<nblk, AFM_RELAX_THREADS, 0, (cudaStream_t)stream>>>(P);
+    else relax_afm_kernel<false><<<nblk, AFM_RELAX_THREADS, 0, (cudaStream_t)stream>>>(P);
     PPGPU_CHECK_LAUNCH("relax_afm_kernel");
     return set_ok();
 }

@@ -74,45 +74,39 @@ __device__ __forceinline__ dfl spline_radial_df(const TipSpline &S, dfl x) {
 
 // Force values at the corners of the cell that a stroke was in last, and the cell (-1: none).  A
 // probe stays in its cell for most iterations of a height, and the gathers, 32 lanes in 32
-// places, cost as much of the L1 as the arithmetic costs of the issue slots.
+// places, cost as much of the L1 as the arithmetic costs of the issue slots.  They take 26 registers,
+// a CTA a SM, which only scans of one wave can spare (KEEP_MAX_STROKES in pp_relax.cu).
 struct Corners {
     long long cell;
     float x[8], y[8], z[8];
 };
 
-// Periodic trilinear interpolation of the force (Grid.h:93-111) at the grid coordinate
-// base + u (base integer, u double-float): float32 grid values, double-float weights and
-// compensated sums, so the only rounding left is that of the stored grid values.
-// NC: read-only (non-coherent) gathers; false for a grid written earlier in the same launch.
-template <bool NC = true>
-__device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1, int n2, const int base[3],
-                                                const dfl u[3], dfl F[3], Corners &c) {
-    auto ld = [&](const float4 *q) { return NC ? ldg4(q) : *q; };
-    int ci[3];
+// A point's cell (first corner, wrapped) and its fractions there, t and 1 - t.
+struct CellPoint {
+    int i[3];
     dfl t[3], m[3];
+};
+__device__ __forceinline__ CellPoint cell_point(int n0, int n1, int n2, const int base[3], const dfl u[3]) {
+    CellPoint c;
+    int ci[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        t[k] = split_cell(u[k], ci[k]);
+        c.t[k] = split_cell(u[k], ci[k]);
         ci[k] += base[k];
-        const dfl o = fast_two_sum(1.f, -t[k].h);
-        m[k] = {o.h, __fsub_rn(o.l, t[k].l)};
+        const dfl o = fast_two_sum(1.f, -c.t[k].h);
+        c.m[k] = {o.h, __fsub_rn(o.l, c.t[k].l)};
     }
-    const int ix0 = wrap_index(ci[0], n0), iy0 = wrap_index(ci[1], n1), iz0 = wrap_index(ci[2], n2);
-    const long long r00 = ((long long)ix0 * n1 + iy0) * n2;
-    if (r00 + iz0 != c.cell) {
-        c.cell = r00 + iz0;
-        const long long dx = ix0 + 1 == n0 ? -(long long)ix0 * n1 * n2 : (long long)n1 * n2;
-        const long long dy = iy0 + 1 == n1 ? -(long long)iy0 * n2 : (long long)n2;
-        const int dz = iz0 + 1 == n2 ? -iz0 : 1;
-        // corner order (x, y, z bits): 000 001 010 011 100 101 110 111
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float4 v = ld(FE + c.cell + ((k & 4) ? dx : 0) + ((k & 2) ? dy : 0) + ((k & 1) ? dz : 0));
-            c.x[k] = v.x;
-            c.y[k] = v.y;
-            c.z[k] = v.z;
-        }
-    }
+    c.i[0] = wrap_index(ci[0], n0);
+    c.i[1] = wrap_index(ci[1], n1);
+    c.i[2] = wrap_index(ci[2], n2);
+    return c;
+}
+
+// The interpolated force from the corners' values v(corner, component); corner order (x, y, z
+// bits): 000 001 010 011 100 101 110 111.
+template <class Value>
+__device__ __forceinline__ void cell_force(const CellPoint &c, Value v, dfl F[3]) {
+    const dfl *m = c.m, *t = c.t;
     const dfl wxy[4] = {df_mul(m[0], m[1]), df_mul(m[0], t[1]), df_mul(t[0], m[1]), df_mul(t[0], t[1])};
     dfl w[8];
 #pragma unroll
@@ -125,9 +119,9 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
         dfl p[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const float v = comp == 0 ? c.x[k] : (comp == 1 ? c.y[k] : c.z[k]);
-            p[k] = two_prod(w[k].h, v);
-            p[k].l = __fmaf_rn(w[k].l, v, p[k].l);
+            const float f = v(k, comp);
+            p[k] = two_prod(w[k].h, f);
+            p[k].l = __fmaf_rn(w[k].l, f, p[k].l);
         }
         const dfl a0 = df_add_raw(p[0], p[1]), a1 = df_add_raw(p[2], p[3]);
         const dfl a2 = df_add_raw(p[4], p[5]), a3 = df_add_raw(p[6], p[7]);
@@ -135,13 +129,48 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
         F[comp] = two_sum(r.h, r.l);
     }
 }
-// The same, gathering every time.
+
+// Periodic trilinear interpolation of the force (Grid.h:93-111) at the grid coordinate
+// base + u (base integer, u double-float): float32 grid values, double-float weights and
+// compensated sums, so the only rounding left is that of the stored grid values.
+// NC: read-only (non-coherent) gathers; false for a grid written earlier in the same launch.
 template <bool NC = true>
 __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1, int n2, const int base[3],
                                                 const dfl u[3], dfl F[3]) {
-    Corners c;
-    c.cell = -1;
-    interp_force_df<NC>(FE, n0, n1, n2, base, u, F, c);
+    auto ld = [&](const float4 *q) { return NC ? ldg4(q) : *q; };
+    const CellPoint p = cell_point(n0, n1, n2, base, u);
+    const int ix0 = p.i[0], iy0 = p.i[1], iz0 = p.i[2];
+    const int ix1 = (ix0 + 1 == n0) ? 0 : ix0 + 1;
+    const int iy1 = (iy0 + 1 == n1) ? 0 : iy0 + 1;
+    const int iz1 = (iz0 + 1 == n2) ? 0 : iz0 + 1;
+    const long long r00 = ((long long)ix0 * n1 + iy0) * n2, r01 = ((long long)ix0 * n1 + iy1) * n2;
+    const long long r10 = ((long long)ix1 * n1 + iy0) * n2, r11 = ((long long)ix1 * n1 + iy1) * n2;
+    const float4 c[8] = {ld(FE + r00 + iz0), ld(FE + r00 + iz1), ld(FE + r01 + iz0), ld(FE + r01 + iz1),
+                         ld(FE + r10 + iz0), ld(FE + r10 + iz1), ld(FE + r11 + iz0), ld(FE + r11 + iz1)};
+    cell_force(p, [&](int k, int comp) { return comp == 0 ? c[k].x : (comp == 1 ? c[k].y : c[k].z); }, F);
+}
+// The same, gathering when the stroke has left its cell.
+template <bool NC = true>
+__device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1, int n2, const int base[3],
+                                                const dfl u[3], dfl F[3], Corners &c) {
+    auto ld = [&](const float4 *q) { return NC ? ldg4(q) : *q; };
+    const CellPoint p = cell_point(n0, n1, n2, base, u);
+    const int ix0 = p.i[0], iy0 = p.i[1], iz0 = p.i[2];
+    const long long r00 = ((long long)ix0 * n1 + iy0) * n2;
+    if (r00 + iz0 != c.cell) {
+        c.cell = r00 + iz0;
+        const long long dx = ix0 + 1 == n0 ? -(long long)ix0 * n1 * n2 : (long long)n1 * n2;
+        const long long dy = iy0 + 1 == n1 ? -(long long)iy0 * n2 : (long long)n2;
+        const int dz = iz0 + 1 == n2 ? -iz0 : 1;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float4 v = ld(FE + c.cell + ((k & 4) ? dx : 0) + ((k & 2) ? dy : 0) + ((k & 1) ? dz : 0));
+            c.x[k] = v.x;
+            c.y[k] = v.y;
+            c.z[k] = v.z;
+        }
+    }
+    cell_force(p, [&](int k, int comp) { return comp == 0 ? c.x[k] : (comp == 1 ? c.y[k] : c.z[k]); }, F);
 }
 
 // interp_force_df split over a group of TPS lanes (TPS in {1, 2, 4, 8}, groups aligned in the
@@ -152,22 +181,15 @@ __device__ __forceinline__ void interp_force_df(const float4 *FE, int n0, int n1
 // result bit for bit.
 template <int TPS, bool NC = true>
 __device__ __forceinline__ void interp_force_df_group(const float4 *FE, int n0, int n1, int n2, const int base[3],
-                                                      const dfl u[3], dfl F[3], int sub, unsigned mask, Corners &corners) {
+                                                      const dfl u[3], dfl F[3], int sub, unsigned mask) {
     if constexpr (TPS == 1) {
-        interp_force_df<NC>(FE, n0, n1, n2, base, u, F, corners);
+        interp_force_df<NC>(FE, n0, n1, n2, base, u, F);
     } else {
         constexpr int CPL = 8 / TPS;  // corners per lane
         auto ld = [&](const float4 *q) { return NC ? ldg4(q) : *q; };
-        int ci[3];
-        dfl t[3], m[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            t[k] = split_cell(u[k], ci[k]);
-            ci[k] += base[k];
-            const dfl o = fast_two_sum(1.f, -t[k].h);
-            m[k] = {o.h, __fsub_rn(o.l, t[k].l)};
-        }
-        const int ix0 = wrap_index(ci[0], n0), iy0 = wrap_index(ci[1], n1), iz0 = wrap_index(ci[2], n2);
+        const CellPoint p0 = cell_point(n0, n1, n2, base, u);
+        const dfl *t = p0.t, *m = p0.m;
+        const int ix0 = p0.i[0], iy0 = p0.i[1], iz0 = p0.i[2];
         const int ix1 = (ix0 + 1 == n0) ? 0 : ix0 + 1;
         const int iy1 = (iy0 + 1 == n1) ? 0 : iy0 + 1;
         const int iz1 = (iz0 + 1 == n2) ? 0 : iz0 + 1;

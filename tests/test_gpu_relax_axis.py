@@ -130,3 +130,55 @@ def test_afm_axis_matches_one_lane(gpulib, npix, nz):
         assert x[:npix].equal(y)
     it = one[2][:npix]
     assert int((it.clamp(max=127) + 1).sum()) == total
+
+
+TILTED = np.array([[6.8, 0, 0], [0.9, 5.8, 0], [0.4, -0.5, 8.2]])
+
+
+@pytest.mark.parametrize("spline", [False, True])
+@pytest.mark.parametrize("cell", [CELL, TILTED], ids=["diagonal", "tilted"])
+def test_large_scans_match_small_ones(gpulib, cell, spline):
+    """More strokes than keep the corners of their cell (77 824): the same bits as scans of a part of
+    them, one lane a stroke as well."""
+    import torch
+
+    from ppafm_gb300 import device as D
+
+    ff = D.DeviceFF(N, cell, FE=_grid(4).FE)
+    rng = np.random.default_rng(8)
+    xs, ys, zs = rng.uniform(-9, 15, 260), rng.uniform(-9, 15, 301), np.linspace(11.0, 10.0, 4)
+    x = np.linspace(2, 6, 31)
+    with D.tip_spline((x, np.column_stack([-1.25 * (x - 4.0), np.full(31, -1.25)])) if spline else None):
+
+        def run(part):
+            return D.relax_scan(ff, _prm(60), part, ys, zs, df_weights=np.array([1.0, -2.0]), want_iters=True)
+
+        whole = run(xs)
+        parts = [_with_tps(1, lambda p=p: {k: v.clone() for k, v in run(p).items()}) for p in (xs[:130], xs[130:])]
+    for k in whole:
+        assert whole[k].equal(torch.cat([p[k] for p in parts])), k
+
+
+def test_large_afm_scans_match_small_ones(gpulib):
+    """The AFMulator's relaxation beyond 116 736 strokes against a part of them."""
+    import torch
+
+    from ppafm_gb300._lib import AFM_NPARAM, check, dptr, iptr, lib, stream_handle, tptr
+
+    ff = _grid(9)
+    rng = np.random.default_rng(12)
+    many, some, nz = 117001, 60000, 3
+    pts = torch.tensor(np.column_stack([rng.uniform(-9, 15, (many, 2)), rng.uniform(3, 12, many), np.zeros(many)]).astype(np.float32)).cuda()
+    prm = np.zeros(AFM_NPARAM)
+    prm[0:2], prm[4:8], prm[8:12] = (0.5, 0.1), np.array([0.25, 0.25, 0.0, 30.0]) / -16.0217662, (0.1, 0.0, -2.998, 3.0)
+    prm[12:24] = [1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, -0.1]
+    inv = np.ascontiguousarray(np.linalg.inv(CELL).T)
+    W = np.array([1.0, -2.0])
+
+    def run(m):
+        o = [torch.full((m, nz, 4), 9.0, device="cuda"), torch.full((m, nz, 4), 9.0, device="cuda"), torch.zeros((m, nz), dtype=torch.int32, device="cuda"), torch.full((m, nz - 1), 9.0, device="cuda")]
+        check(lib().ppgpu_relax_afm(tptr(ff.FE), iptr(np.array(N, np.int32)), dptr(inv), dptr(prm), m, tptr(pts), nz, tptr(o[0]), tptr(o[1]), tptr(o[2]), 2, dptr(W), tptr(o[3]), None, stream_handle()))
+        return o
+
+    for x, y in zip(run(many), run(some)):
+        assert x[:some].equal(y)
