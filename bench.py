@@ -139,14 +139,28 @@ def read_measured_peaks():
         return {}
 
 
-def ff_bytes_roofline(name, moved, t_ff):
-    """Roofline of a force field summed by boxes: the bytes it cannot do without (each grid point
-    written, each atom read once) against the measured copy rate.  The pairs it sums are 1/15 (a small
-    molecule) to 1/130 (the slab) of the direct sum's, so the direct sum's flops say nothing here; it
-    is bound by instruction issue."""
+def bytes_floor_roofline(name, bound, moved, t, traffic):
+    """Roofline of a kernel that neither memory nor the FMA pipe bounds: the bytes it cannot do without
+    against the measured copy rate, as a floor, beside what bounds it (ncu).  Force fields by boxes:
+    each grid point written, each atom read once; the pairs they sum are 1/15 (a small molecule) to 1/130
+    (the slab) of the direct sum's, whose flops say nothing here.  Relaxations: the rows of the grid that
+    the probe visits read once, 32 B out a pixel height."""
     hbm = read_measured_peaks().get("hbm_gbs")
-    achieved, peak = moved / t_ff / 1e9, hbm or 6800.0
-    return {"bound": "hbm", "kernel": name, "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs" if hbm else "fallback 6800 GB/s", "bytes_per_launch": moved}
+    achieved, peak = moved / t / 1e9, hbm or 6800.0
+    return {"bound": bound, "kernel": name, "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": ("MEASURED_PEAKS.json hbm_gbs" if hbm else "fallback 6800 GB/s") + "; achieved counts the floor's bytes", "bytes_per_launch": moved, "traffic": traffic}
+
+
+ISSUE = "instruction issue"
+
+
+def ff_route(n, cell, natoms, ncharged, mode):
+    """(nodes per axis, levels above the leaves) of a force field by boxes; (0, 0): pair by pair."""
+    from ppafm_gb300._lib import check, dptr, iptr, lib
+
+    out = np.zeros(2, np.int32)
+    nn, c = np.array(n, np.int32), np.ascontiguousarray(cell, dtype=np.float64)
+    check(lib().ppgpu_ff_route(iptr(nn), dptr(c), iptr(nn), natoms, ncharged, mode, 0, None, None, 0, iptr(out)))
+    return int(out[0]), int(out[1])
 
 
 def ffma_peak_tflops(torch, lib, check, tptr, stream_handle):
@@ -183,8 +197,13 @@ class PointChargeJob:
         self.npts = int(np.prod(self.pl.gridN))
         self.natoms = self.pl.natoms
         self.nch = self.pl.ncharged
-        self.ff_name = "ff_box_kernel<LJC> and box_up_kernel (force field by boxes)" if self.pl.Q != 0.0 else "ff_box_kernel<LJ> and box_up_kernel (force field by boxes)"
-        self.launches_per_step = 3 if self.natoms < 5000 else 5  # the leaves, one or three levels of boxes above them, relax
+        from ppafm_gb300._lib import FF_LJ, FF_LJC
+
+        lj = self.pl.Q == 0.0
+        nodes, levels = ff_route(self.pl.gridN, self.pl.lvec[1:4], self.natoms, 0 if lj else self.nch, FF_LJ if lj else FF_LJC)
+        kind = "LJ" if lj else "LJC"
+        self.ff_name = f"ff_box_kernel<{kind}> and box_up_kernel (force field by boxes, {nodes} nodes an axis, {levels} levels above the leaves)" if nodes else f"ff_kernel<{kind}> (force field pair by pair)"
+        self.launches_per_step = 1 + (levels if nodes else 0) + 1 + (1 if lj else 0)  # the field (leaves, levels above them), its clamp after LJ alone, relax
         self.pinned_slots(2)
         self.host_in = {k: np.asarray(w[k]).copy() for k in ("Zs", "Rs", "Qs")}
 
@@ -209,7 +228,7 @@ class PointChargeJob:
         self.pl.atoms.copy_(self.rec_pinned[slot], non_blocking=True)
 
     def ff_roofline(self, t_ff):
-        return ff_bytes_roofline(self.ff_name, 16.0 * self.npts + 48.0 * self.natoms, t_ff)
+        return bytes_floor_roofline(self.ff_name, ISSUE, 16.0 * self.npts + 48.0 * self.natoms, t_ff, read_profile_traffic("ff_box_kernel", self.w["name"]))
 
     def config(self):
         return {"atoms": len(self.w["Zs"]), "atoms_with_images": self.natoms, "charged_atoms_with_images": self.nch}
@@ -227,7 +246,7 @@ class OverlapJob:
         self.torch = torch
         self.pl = HL.DensityOverlapPipeline.from_workload(w, relax=relax, want_iters=False)
         self.npts = int(np.prod(self.pl.gridN))
-        self.launches_per_step = 12  # 2 x (sums + power), 4 R2C, spectra, C2R x4, pack, relax (cuFFT launches counted as one each)
+        self.launches_per_step = 11  # 2 x (clip, power and sums), 4 R2C, spectra, C2R x4, pack, C2R of V, relax (cuFFT launches counted as one each)
         self.host = [torch.empty(self.pl.gridN, dtype=torch.float32, pin_memory=True) for _ in range(3)]
         for h, d in zip(self.host, (self.pl.rho_s, self.pl.rho_q, self.pl.rho_t)):
             h.copy_(d)
@@ -590,8 +609,8 @@ def run_ours(args, rank, world, local):
         if world > 1:
             torch.distributed.barrier()
 
-    # ---------------- device-resident steps, pipelined: step k+1's force field runs while step
-    # k's relaxation finishes (force-field grids and output sets in flight,
+    # ---------------- device-resident steps, pipelined: step k+1's force field starts behind step
+    # k's relaxation and fills the SMs that it leaves idle (force-field grids and output sets in flight,
     # HighLevel.StepPipeline).  A force field that fits in L2 is flushed from it before every
     # timed step's relaxation: 256 MB written on the relaxation stream once the step's force
     # field is done, so the relaxation reads its grid from DRAM, not from the L2 lines its
@@ -706,22 +725,20 @@ def run_ours(args, rank, world, local):
         return None
 
     # ---------------- roofline of the dominant kernel
+    c = pl.lvec[1:4]  # scans of up to 30 000 strokes on an orthogonal cell: a lane for each axis
+    relax_lanes = args.relax_tps or (3 if nx * ny <= 30000 and not (c - np.diag(np.diag(c))).any() else 1)
     t_ff_avg = float(np.mean(t_ff))
     t_rx_avg = float(np.mean(t_rx))
     if t_ff_avg >= t_rx_avg and job.ff_roofline(t_ff_avg) is not None:
         roof = job.ff_roofline(t_ff_avg)
-        roof["traffic"] = read_profile_traffic("ff_box_kernel", args.workload)
     else:
-        # relaxation: gathers of 8 float4 corners per FIRE iteration + 32 B out per pixel-z
-        peaks = read_measured_peaks()
-        hbm = peaks.get("hbm_gbs")
-        moved = 128.0 * iters_total / K + 32.0 * units
-        achieved = moved / t_rx_avg / 1e9
-        roof = {"bound": "hbm", "kernel": "relax_kernel<scan> (FIRE + fused df)", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm if hbm else None, "peak_source": "MEASURED_PEAKS.json hbm_gbs" if hbm else "fallback 6800 GB/s", "bytes_per_launch": moved, "traffic": read_profile_traffic("relax_kernel", args.workload)}
-        if not hbm:
-            roof["peak"] = 6800.0
-            roof["frac"] = achieved / 6800.0
+        rows = min(pl.gridN[2], int(np.ptp(pl.zs) / (pl.lvec[3, 2] / pl.gridN[2])) + 8)
+        name = "relax_axis_kernel" if relax_lanes == 3 else "relax_kernel"
+        bound = "a stroke's dependent chain and " + ISSUE
+        roof = bytes_floor_roofline(f"{name}<scan> (FIRE + fused df)", bound, 16.0 * pl.gridN[0] * pl.gridN[1] * rows + 32.0 * units, t_rx_avg, read_profile_traffic(name, args.workload))
 
+    if args.scale != 1.0:
+        roof["traffic"] = None  # measured at full size
     cpu = None
     if not args.no_cpu_baseline and world == 1:
         try:
@@ -744,8 +761,8 @@ def run_ours(args, rank, world, local):
             "probe": {"klat": w["klat"], "krad": w["krad"], "r0": list(w["r0Probe"]), "Q": w["charge"]},
             "df": {"f0": w["f0Cantilever"], "k": w["kCantilever"], "A": w["Amplitude"]},
             "l2": ("inputs larger than L2 (force field %.2f GB)" if npts * 16 >= 129e6 else "force field %.2f GB fits in L2: 256 MB written before every step's relaxation (after its force field) to flush it") % (npts * 16 / 1e9),
-            "relax_lanes_per_stroke": args.relax_tps or 1,
-            "steps": "pipelined: step k+1's force field runs while step k's relaxation finishes (three force-field grids and output sets in flight, relaxations on a higher-priority stream); stage_ms are each kernel's own event-timed duration on its stream",
+            "relax_lanes_per_stroke": relax_lanes,
+            "steps": "pipelined: step k+1's force field starts behind step k's relaxation, whose blocks go first, and fills the SMs that it leaves idle; where both fill the GPU their times add up (three force-field grids and output sets in flight, relaxations on a higher-priority stream); stage_ms are each kernel's own event-timed duration on its stream",
             "parallelism": f"replicas x{world}",
         }
     )
@@ -942,8 +959,7 @@ def run_afmulator(args, rank, world, local):
     _lib.check(L.ppgpu_device_status(_lib.stream_handle()))
     npts = int(np.prod(afm.nDim))
     natoms = float(np.mean([len(z) for _, _, z, _, _ in seen]))
-    roof = ff_bytes_roofline("ff_box_kernel<QZS> (LJ + point-charge tip force field by boxes)", 16.0 * npts + 48.0 * natoms, t_ff)
-    roof["traffic"] = read_profile_traffic("ff_box_kernel", "afmulator")
+    roof = bytes_floor_roofline("ff_box_kernel<QZS> (LJ + point-charge tip force field by boxes)", ISSUE, 16.0 * npts + 48.0 * natoms, t_ff, read_profile_traffic("ff_box_kernel", "afmulator"))
     if rank != 0:
         return None
     cpu = None

@@ -172,7 +172,8 @@ int ppgpu_set_tip_spline(int n, const double *xs, const double *ydys);
 /* Lanes per stroke of ppgpu_relax_strokes / ppgpu_relax_scan (no reference counterpart):
  * tps 1, 2, 4 or 8 lanes share each stroke's trilinear gathers (same results bit for bit);
  * 0 restores the default: 1, or, on scans too small to fill the GPU, a lane for each axis of a
- * stroke (same results again).  ppgpu_get_relax_tps returns the value used for nstroke strokes. */
+ * stroke (same results again).  ppgpu_get_relax_tps returns the lanes that share a stroke's gathers: 1 by
+ * default, also where a stroke has a lane for each axis. */
 int ppgpu_set_relax_tps(int tps);
 /* No counterpart in the reference (a launch-shape knob).  Threads per CTA of the single-grid
  * force-field kernel: 128 or 256, 0 = the default (128). Only for fields

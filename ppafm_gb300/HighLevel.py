@@ -395,7 +395,7 @@ class StepPipeline:
     another, of higher priority.  A force field starts just behind the relaxation of the step
     before, whose blocks are placed first, evenly, and fills the SMs around them: a relaxation that
     found the SMs taken got its blocks as they became free, more on some SMs than on others, and
-    took 2.07 instead of 1.27 ms on the small molecule (a step 2.13 -> 1.47 ms).  Step k's force
+    took 2.07 instead of 1.27 ms on the small molecule (a step 2.14 -> 1.49 ms).  Step k's force
     field also waits for the relaxation that last read its grid (and for ``after``, e.g. the copy of the
     step's inputs); step k's
     relaxation waits for its force field and for ``release``d events on its output set (e.g.

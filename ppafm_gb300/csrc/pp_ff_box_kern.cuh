@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(BOX_NT, 2) box_up_kernel(const __grid_constant
     if (warp == 0 && lane < 3 * N) box_node_table<N>(prm, B, level, b, lane, s_node, s_off);
     for (int i = tid; i < Cols::ACC * C4; i += NT) own[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    auto weights = [&]() {  // by the warp that has no nodes
+    auto weights = [&]() {  // by the last warp, which has no node columns with 10 nodes
         for (int i = lane; i < 6 * N; i += 32) {
             const int a = i / (2 * N), c = i / N % 2, n = i % N;
             dfl x;
@@ -254,8 +254,7 @@ __global__ void __launch_bounds__(BOX_NT, 2) box_up_kernel(const __grid_constant
                 cheb_row<N>(x, [&](int k, dfl w) { s_w[a][c][k][n] = df_round(w); });
         }
     };
-    // ---- far atoms on the nodes: thread = node column (ia, ib), one of two parts of the atoms; 200
-    // threads, in 7 of the 8 warps
+    // ---- far atoms on the nodes: thread = node column (ia, ib), one of SUBS parts of the atoms
     const int sub = tid / N2, col = tid % N2;
     BoxSums<MODE, WITH_E, P2N> M;
     M.zero();
