@@ -71,10 +71,11 @@ struct ChebNodes {
     }
 };
 
-// Weights [points of the axis][point][node] of evenly spaced points over [-1, 1].
-template <int N>
+// Weights [points of the axis][point][node] of evenly spaced points over [-1, 1]; LOW: what float32
+// leaves of them.
+template <int N, bool LOW>
 struct ChebPoints {
-    float w[BOX_S + 1][BOX_S][N] = {}, l[BOX_S + 1][BOX_S][N] = {};  // high and low parts
+    float w[BOX_S + 1][BOX_S][N] = {};
     constexpr ChebPoints() {
         constexpr ChebNodes<N> c;
         for (int m = 1; m <= BOX_S; m++)
@@ -84,15 +85,14 @@ struct ChebPoints {
                     double p = c.w[k];
                     for (int j = 0; j < N; j++)
                         if (j != k) p *= x - c.t[j];
-                    w[m][i][k] = (float)p;
-                    l[m][i][k] = (float)(p - (double)w[m][i][k]);
+                    w[m][i][k] = LOW ? (float)(p - (double)(float)p) : (float)p;
                 }
     }
 };
-static __device__ const ChebPoints<8> c_points8 = ChebPoints<8>();
-static __device__ const ChebPoints<10> c_points10 = ChebPoints<10>();
+static __device__ const ChebPoints<8, false> c_points8 = ChebPoints<8, false>();
+static __device__ const ChebPoints<10, false> c_points10 = ChebPoints<10, false>();
 template <int N>
-__device__ __forceinline__ const ChebPoints<N> &cheb_points() {
+__device__ __forceinline__ const ChebPoints<N, false> &cheb_points() {
     if constexpr (N == 8) return c_points8;
     else return c_points10;
 }

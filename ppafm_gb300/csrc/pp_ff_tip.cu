@@ -182,6 +182,7 @@ constexpr double TIP_KAPPA = 5.0;
 constexpr int TIP_NT = 256;
 constexpr int TIP_N = 10, TIP_N2 = 100, TIP_N3 = 1000;  // nodes
 constexpr int TIP_X = 4;  // of the box's x in the plane
+static __device__ const ChebPoints<TIP_N, true> c_points_low = ChebPoints<TIP_N, true>();
 
 // acc += w v (both double-floats).
 __device__ __forceinline__ void df_fma(dfl &acc, dfl w, dfl v) { df_acc(acc, df_mul_raw(w, v)); }
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
     for (int i = tid; i < 3 * XS * TIP_N; i += NT) {
         const int a = i / (XS * TIP_N), pt = (i / TIP_N) % XS, k = i % TIP_N;
         const int m = (a == 0 ? hi[0] - lo[0] : (a == 1 ? hi[1] - lo[1] : hi[2] - lo[2])) + 1;
-        (a == 0 ? s_wx : (a == 1 ? s_wy : s_wz))[pt][k] = {cheb_points<TIP_N>().w[m][pt][k], cheb_points<TIP_N>().l[m][pt][k]};
+        (a == 0 ? s_wx : (a == 1 ? s_wy : s_wz))[pt][k] = {cheb_points<TIP_N>().w[m][pt][k], c_points_low.w[m][pt][k]};
     }
     __syncthreads();
 
