@@ -672,8 +672,11 @@ __global__ void __launch_bounds__(BOX_NT, 2) ff_box_kernel(const __grid_constant
                     for (int k = 0; k < 3; k++)
                         q[k] = ((prm.dA[k] * (prm.i0[0] + lo[0] + x)) + prm.dB[k] * (prm.i0[1] + lo[1] + y)) +
                                prm.dC[k] * (prm.i0[2] + lo[2] + 2 * i + h);
+                    // The far sums are finite, unless an atom overflows them (a charge of infinity, a tip's
+                    // charges beside an atom beyond 1e19 A): all atoms then.
+                    bool near_only = listed;
+                    float far[8] = {};  // component k of the far sums, from the lines again
                     if (listed) {
-                        float far[8] = {};  // component k of the far sums, from the lines again
 #pragma unroll 1
                         for (int k = 0; k < NC; k++) {
                             float v = 0.f;
@@ -684,7 +687,10 @@ __global__ void __launch_bounds__(BOX_NT, 2) ff_box_kernel(const __grid_constant
                                          reinterpret_cast<const float *>(line)[(k * XS + x) * N2 + (c0 >> 1) * 2 * N + 2 * y0 + (c0 & 1)], v);
                             }
                             far[k < NC1 ? k : k - NC1 + 4] = v;
+                            near_only = near_only && fabsf(v) <= 3.4e38f;
                         }
+                    }
+                    if (near_only) {
                         f = box_point_slow<MODE, WITH_E>(prm, df_from(q[0]), df_from(q[1]), df_from(q[2]), s_near, wide, nnear, nch,
                                                          make_float4(far[0], far[1], far[2], far[3]),
                                                          make_float4(far[4], far[5], far[6], far[7]));

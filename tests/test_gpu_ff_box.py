@@ -176,6 +176,64 @@ def test_atoms_without_attraction_are_far(gpulib):
     assert ms[1] < 8.0 * ms[0], ms
 
 
+@pytest.mark.parametrize("mode", ["lj", "ljc", "coulomb"])
+def test_an_atom_beyond_float32_adds_nothing(gpulib, mode):
+    """An atom at 1e20 A, whose r^2 overflows: the bits of the field with that atom at 1e19 A, whose
+    force is below float32's least."""
+    from ppafm_gb300 import device as D
+
+    n = (113, 129, 97)
+    cell = np.diag(np.array(n) * 0.1)
+    R, c, q = _atoms(np.random.default_rng(31), 300, cell, "plane")
+    M = dict(ljc=D.FF_LJC, lj=D.FF_LJ, coulomb=D.FF_COULOMB)[mode]
+    got = []
+    for x in (1e19, 1e20):
+        R[11] = (x, 0.0, 0.0)
+        rec, na, nch = D.pack_atoms(R, None if mode == "coulomb" else c, None if mode == "lj" else q)
+        got.append(D.DeviceFF(n, cell).compute(rec, na, nch, M, Q=-0.05 if mode == "ljc" else 0.0).FE.clone())
+    assert bool(got[0].isfinite().all()) and got[1].equal(got[0])
+
+
+def test_tip_charges_and_an_atom_beyond_float32(gpulib):
+    """The same with a tip's charges, whose differences overflow there: every point goes through all atoms,
+    as pair by pair (a small sub-box), bit for bit."""
+    from ppafm_gb300 import device as D
+
+    n = (113, 129, 97)
+    cell = np.diag(np.array(n) * 0.1)
+    R, c, q = _atoms(np.random.default_rng(33), 100, cell, "plane")
+    R[11] = (1e20, 0.0, 0.0)
+    tip = dict(Qs=[-10.0, 20.0, -10.0, 0.0], QZs=[0.1, 0.0, -0.1, 0.0])
+    rec, na, nch = D.pack_atoms(R, c, q)
+    ff = D.DeviceFF(n, cell)
+    g = ff.compute(rec, na, nch, D.FF_QZS, with_E=True, **tip).grid4.cpu().numpy().astype(np.float64)
+    assert np.isfinite(g).all()
+    for i0 in [(0, 0, 0), (50, 60, 40), (107, 124, 88)]:
+        ref = _subgrid_f64(ff, i0, (6, 5, 9), rec, na, nch, D.FF_QZS, 0.0, 0.0, D.FF_WITH_E, tip)
+        assert (g[i0[0] : i0[0] + 6, i0[1] : i0[1] + 5, i0[2] : i0[2] + 9] == ref).all()
+
+
+def test_infinite_charge_as_pair_by_pair(gpulib):
+    """The same infinities and NaNs as the direct sum's (a small sub-box), bit for bit elsewhere too: all
+    points take its slow path."""
+    import torch
+
+    from ppafm_gb300 import device as D
+
+    n = (113, 129, 97)
+    cell = np.diag(np.array(n) * 0.1)
+    R, _, q = _atoms(np.random.default_rng(32), 300, cell, "plane")
+    q[7] = np.inf
+    R[7] = (300.0, 2.0, 5.0)
+    rec, na, nch = D.pack_atoms(R, None, q)
+    ff = D.DeviceFF(n, cell)
+    g = ff.compute(rec, na, nch, D.FF_COULOMB, with_E=True).grid4
+    for i0 in [(0, 0, 0), (50, 60, 40), (107, 124, 88)]:
+        ref = ff.compute_subgrid(i0, (6, 5, 9), rec, na, nch, D.FF_COULOMB, with_E=True).view(6, 5, 9, 4)
+        got = g[i0[0] : i0[0] + 6, i0[1] : i0[1] + 5, i0[2] : i0[2] + 9]
+        assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.nan_to_num(nan=0.0), ref.nan_to_num(nan=0.0))
+
+
 def _subgrid_f64(ff, i0, ns, rec, na, nch, mode, Q, Fmax, flags, tip):
     """A sub-box of the grid in float64 (compute_subgrid has no tip charges)."""
     import torch
