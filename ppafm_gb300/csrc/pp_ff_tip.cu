@@ -74,6 +74,27 @@ struct TipSums {
     }
 };
 
+// A part of an atom record (k: 0 x, y; 1 z; 2 charge) with finite coordinates (and their low parts) of
+// 1e18 A at most: from there on a charge's field is nothing in float32, and r^2 would overflow.
+__device__ __forceinline__ float4 tip_record(float4 v, int k) {
+    auto lim = [](float &h, float &l) {
+        if (!(fabsf(h) > 1e18f && fabsf(h) <= 3.4e38f)) return;
+        h = copysignf(1e18f, h);
+        l = 0.f;
+    };
+    if (k == 0) {
+        lim(v.x, v.z);
+        lim(v.y, v.w);
+    } else if (k == 1) {
+        lim(v.x, v.y);
+    }
+    return v;
+}
+__device__ __forceinline__ void tip_limit(float4 *record) {
+    record[0] = tip_record(record[0], 0);
+    record[1] = tip_record(record[1], 1);
+}
+
 // Adds a charge q (negated coordinates in r0, r1) to the sums at positions p (x and y of the first
 // one only when ORTHO).
 template <int KIND, bool WITH_E, bool ORTHO>
@@ -154,7 +175,7 @@ __global__ void __launch_bounds__(TIP_THREADS, 4) ff_tip_kernel(const FFParams p
     for (int base = 0; base < prm.ncharged; base += FF_TILE) {
         const int nj = min(FF_TILE, prm.ncharged - base);
         __syncthreads();
-        for (int i = tid; i < nj * FF_REC; i += TIP_THREADS) s_at[i] = prm.atoms[(size_t)base * FF_REC + i];
+        for (int i = tid; i < nj * FF_REC; i += TIP_THREADS) s_at[i] = tip_record(prm.atoms[(size_t)base * FF_REC + i], i % FF_REC);
         __syncthreads();
         for (int j = 0; j < nj; j++) tip_add<KIND, WITH_E, ORTHO>(p, s_at[3 * j], s_at[3 * j + 1], s_at[3 * j + 2].z, S);
         S.fold<WITH_E>();
@@ -265,6 +286,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_up_kernel(const __grid_constant
         if (i < last) {
             j0 = nlist >= 0 ? (int)*share_list<TIP_N, NC>(share, i) : i;
             box_gather(prm, tile + tid * FF_REC, j0);
+            tip_limit(tile + tid * FF_REC);
         }
         box_pick<M_COUL, TIP_N, NT>(B, pk, level, nanc, tile, min(NT, last - i0), 1, true, nmid, nzero, place);
         if (place >= 0 && nleft + place < BOX_LEFT) s_left[nleft + place] = (unsigned short)j0;
@@ -395,6 +417,7 @@ __global__ void __launch_bounds__(TIP_NT, 2) tip_box_kernel(const __grid_constan
         if (i < (all ? nat : ncand)) {
             j = all || nlist < 0 ? i : (int)*share_list<TIP_N, NC>(share, i);
             box_gather(prm, tiles + ((t & 1) * NT + tid) * FF_REC, j);
+            tip_limit(tiles + ((t & 1) * NT + tid) * FF_REC);
         }
         return j;
     };

@@ -143,3 +143,24 @@ def test_tip_boxes_wide_indices(gpulib, kind):
         tol = 2.0**-23 * np.abs(ref) + np.column_stack([floor, floor, floor, floor_E])
         d = np.abs(g - ref)
         assert (d <= tol).all(), (i0, float((d / tol).max()))
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("n", [(9, 14, 33), (113, 97, 130)], ids=["pairs", "boxes"])
+def test_a_charge_beyond_float32_adds_nothing(gpulib, kind, n):
+    """A charge at 1e20 A, whose r^2 overflows float32: the bits of the field of the others, in place of
+    the first charge's record a second one that is too far to show."""
+    import torch
+
+    from ppafm_gb300 import device as D
+
+    rng = np.random.default_rng(77)
+    cell = np.diag(np.array(n) * 0.1)
+    R = np.column_stack([rng.uniform(-4, 15, 200), rng.uniform(-4, 15, 200), rng.uniform(-3, -0.5, 200)])
+    q = rng.uniform(-0.3, 0.3, 200) * 14.399645
+    got = []
+    for far in (1e16, 1e20, -3e37):  # at 1e16 A q / r^3 is below float32's least as well
+        R[11] = (far, 0.3 * far, 0.0)
+        rec, na, nch = D.pack_atoms(R, None, q)
+        got.append(D.DeviceFF(n, cell).compute(rec, na, nch, D.FF_COULOMB, kind=kind, with_E=True).FE.clone())
+    assert torch.isfinite(got[0]).all() and got[1].equal(got[0]) and got[2].equal(got[0])
